@@ -118,152 +118,67 @@ __device__ __forceinline__ void srnh(double hu_l, double hu_r, double hv_l, doub
   flux[4] = As * xi * n0 * unew * uv / w3 + As * xi * n1 * vnew * uv / w3;
 }
 
-// SRNH flux specialised to manapy's constant As = 0 (d = 0, beta = 0): every
-// term multiplied by those zeros is dropped and flux[4] is identically zero.
-// For finite inputs this changes no rounding: dropped terms are signed zeros
-// added to sums, and sign_k * x / sigma equals sign_k * (x / sigma) exactly
-// because sign_k is +-1 or 0.  FAST additionally takes the eigenvalues of
-// manapy's cubic in closed form ({0, u+c, u-c}, ordered as the trigonometric
-// formula orders them) and replaces divisions by a shared denominator with
-// one reciprocal: results then differ from manapy by rounding only.
-template <bool FAST>
+// SRNH flux specialised to manapy's constant As = 0 (d = 0, beta = 0; flux[4] is identically
+// zero), with the eigenvalues of manapy's cubic lambda (lambda^2 - 2 u lambda + u^2 - c^2) in
+// closed form, a = u + c, b = u - c and 0.  Put into manapy's rows
+//   r_k = sum_k sign(lambda_k) {gamma, alpha sums, c^2} / sigma_k
+// they cancel: with l' the other two eigenvalues sigma_k = +-(lambda_k - l')(lambda_k - l''),
+// gamma_k = c^2 - u^2 + l' l'' and c^2 - u^2 = -a b, so for lambda = a, b the three quotients
+// are -b / 2c, -1 / 2c, c / 2a and a / 2c, 1 / 2c, -c / 2b; lambda = 0 has sign 0.  Rows 2
+// and 3 (tangential velocity, tracer) are v and c_h times row 0 plus the wave of speed u.
+// Results differ from manapy's by rounding only.
+//
+// The FP64 pipe bounds the face kernels (about 500 FP64 instructions per face when written
+// row by row, with 9 divisions), so quotients that share a denominator, or whose
+// denominators may be multiplied, take one division: 1 / (sl sr (sl + sr)) for the Roe means
+// (hu_l / h_l sl = hu_l / sl), 1 / (2 c a b) for 1 / 2c, 1 / a and 1 / b, 1 / w_h.
 __device__ __forceinline__ void srnh0(double hu_l, double hu_r, double hv_l, double hv_r, double h_l, double h_r,
                                       double hc_l, double hc_r, double Z_l, double Z_r, double n0, double n1,
-                                      double mesure, double grav, double flux[4]) {
-  const double ninv0 = -1 * n1, ninv1 = n0;
+                                      double im, double grav, double flux[4]) {
+  // im: 1 / mesure
   const double sl = sqrt(h_l), sr = sqrt(h_r);
-  double u_h, v_h, c_h, un_h, vn_h, uleft, vleft, uright, vright;
-  if (FAST) {
-    const double il = 1 / h_l, ir = 1 / h_r, is = 1 / (sl + sr), im = 1 / mesure;
-    u_h = (hu_l * il * sl + hu_r * ir * sr) * is;
-    v_h = (hv_l * il * sl + hv_r * ir * sr) * is;
-    c_h = (hc_l * il * sl + hc_r * ir * sr) * is;
-    un_h = (u_h * n0 + v_h * n1) * im;
-    vn_h = (u_h * ninv0 + v_h * ninv1) * im;
-    uleft = (hu_l * n0 + hv_l * n1) * im;
-    vleft = (hu_l * ninv0 + hv_l * ninv1) * im;
-    uright = (hu_r * n0 + hv_r * n1) * im;
-    vright = (hu_r * ninv0 + hv_r * ninv1) * im;
-  } else {
-    u_h = (hu_l / h_l * sl + hu_r / h_r * sr) / (sl + sr);
-    v_h = (hv_l / h_l * sl + hv_r / h_r * sr) / (sl + sr);
-    c_h = (hc_l / h_l * sl + hc_r / h_r * sr) / (sl + sr);
-    un_h = (u_h * n0 + v_h * n1) / mesure;
-    vn_h = (u_h * ninv0 + v_h * ninv1) / mesure;
-    uleft = (hu_l * n0 + hv_l * n1) / mesure;
-    vleft = (hu_l * ninv0 + hv_l * ninv1) / mesure;
-    uright = (hu_r * n0 + hv_r * n1) / mesure;
-    vright = (hu_r * ninv0 + hv_r * ninv1) / mesure;
-  }
-  const double hroe = (h_l + h_r) / 2, uroe = un_h, vroe = vn_h, croe = c_h;
-  double w_lrh = (h_l + h_r) / 2, w_lrhu = (uleft + uright) / 2, w_lrhv = (vleft + vright) / 2;
-  double w_lrhc = (hc_l + hc_r) / 2;
+  const double K = 1 / (sl * sr * (sl + sr));
+  const double u_h = (hu_l * sr + hu_r * sl) * K;
+  const double v_h = (hv_l * sr + hv_r * sl) * K;
+  const double c_h = (hc_l * sr + hc_r * sl) * K;
+  const double m0 = n0 * im, m1 = n1 * im;   // unit normal; the tangent is (-m1, m0)
+  const double u = u_h * m0 + v_h * m1;
+  const double v = v_h * m0 - u_h * m1;
+  const double uleft = hu_l * m0 + hv_l * m1, vleft = hv_l * m0 - hu_l * m1;
+  const double uright = hu_r * m0 + hv_r * m1, vright = hv_r * m0 - hu_r * m1;
+  const double hroe = (h_l + h_r) / 2;
   const double wd0 = h_r - h_l, wd1 = uright - uleft, wd2 = vright - vleft, wd3 = hc_r - hc_l, wd4 = Z_r - Z_l;
-  const double u2 = uroe * uroe;
-  const double sound = sqrt(grav * hroe);
-  double lambda1, lambda2, lambda3;
-  if (FAST) {
-    // roots of lambda (lambda^2 - 2 u lambda + u^2 - c^2): 0, u + c, u - c; the
-    // trigonometric formula returns the largest, the smallest, then the middle one
-    const double a = uroe + sound, b = uroe - sound;  // a > b
-    const double hi = fmax(a, 0.0), lo = fmin(b, 0.0);
-    lambda1 = hi;
-    lambda2 = lo;
-    lambda3 = (a < 0.0) ? a : ((b > 0.0) ? b : 0.0);
-  } else {
-    const double Q = -(u2 + 3 * grav * hroe) / 9;
-    const double R = uroe * (9 * grav * (2 * hroe) - 2 * u2) / 54;
-    const double theta = acos(R / (sqrt(-(Q * Q * Q))));
-    const double sq = 2 * sqrt(-Q);
-    lambda1 = sq * cos(theta / 3) + (2. / 3) * uroe;
-    lambda2 = sq * cos((theta + 2 * 3.141592653589793) / 3) + (2. / 3) * uroe;
-    lambda3 = sq * cos((theta + 4 * 3.141592653589793) / 3) + (2. / 3) * uroe;
-  }
-  const double alpha1 = lambda1 - uroe, alpha2 = lambda2 - uroe, alpha3 = lambda3 - uroe;
-  const double s2 = sound * sound;
-  const double gamma1 = s2 - u2 + lambda2 * lambda3;
-  const double gamma2 = s2 - u2 + lambda1 * lambda3;
-  const double gamma3 = s2 - u2 + lambda1 * lambda2;
-  const double sigma1 = -alpha1 * alpha2 + alpha2 * alpha3 - alpha1 * alpha3 + (alpha1 * alpha1);
-  const double sigma2 = alpha1 * alpha2 + alpha2 * alpha3 - alpha1 * alpha3 - (alpha2 * alpha2);
-  const double sigma3 = alpha1 * alpha2 - alpha2 * alpha3 - alpha1 * alpha3 + (alpha3 * alpha3);
+  const double c = sqrt(grav * hroe);
+  const double a = u + c, b = u - c;
   const double eps = 1e-10;
-  // lambda / |lambda| is exactly +-1
-  const double sign1 = fabs(lambda1) < eps ? 0. : copysign(1.0, lambda1);
-  const double sign2 = fabs(lambda2) < eps ? 0. : copysign(1.0, lambda2);
-  const double sign3 = fabs(lambda3) < eps ? 0. : copysign(1.0, lambda3);
-  const double sign4 = fabs(uroe) < eps ? 0. : copysign(1.0, uroe);
-  const double sign5 = sign4;
-  const double t1 = (alpha2 + alpha3), t2 = (alpha1 + alpha3), t3 = (alpha1 + alpha2);
-  // |lambda_k| sign_k = lambda_k sign_k exactly
-  const double l1 = lambda1 * sign1, l2 = lambda2 * sign2, l3 = lambda3 * sign3;
-  double g1, g2, g3, q1, q2, q3, lq1, lq2, lq3, vq1, vq2, vq3, cq1, cq2, cq3;
-  double e1, e2, e3, le1, le2, le3, ve1, ve2, ve3, ce1, ce2, ce3;
-  if (FAST) {
-    const double i1 = 1 / sigma1, i2 = 1 / sigma2, i3 = 1 / sigma3;
-    g1 = gamma1 * i1; g2 = gamma2 * i2; g3 = gamma3 * i3;
-    q1 = t1 * i1; q2 = t2 * i2; q3 = t3 * i3;
-    lq1 = l1 * q1; lq2 = l2 * q2; lq3 = l3 * q3;
-    vq1 = vroe * q1; vq2 = vroe * q2; vq3 = vroe * q3;
-    cq1 = croe * q1; cq2 = croe * q2; cq3 = croe * q3;
-    e1 = s2 * i1; e2 = s2 * i2; e3 = s2 * i3;
-    le1 = l1 * e1; le2 = l2 * e2; le3 = l3 * e3;
-    ve1 = vroe * e1; ve2 = vroe * e2; ve3 = vroe * e3;
-    ce1 = croe * e1; ce2 = croe * e2; ce3 = croe * e3;
-  } else {
-    g1 = gamma1 / sigma1; g2 = gamma2 / sigma2; g3 = gamma3 / sigma3;
-    q1 = t1 / sigma1; q2 = t2 / sigma2; q3 = t3 / sigma3;
-    lq1 = (l1 * t1) / sigma1; lq2 = (l2 * t2) / sigma2; lq3 = (l3 * t3) / sigma3;
-    vq1 = (vroe * t1) / sigma1; vq2 = (vroe * t2) / sigma2; vq3 = (vroe * t3) / sigma3;
-    cq1 = (croe * t1) / sigma1; cq2 = (croe * t2) / sigma2; cq3 = (croe * t3) / sigma3;
-    e1 = s2 / sigma1; e2 = s2 / sigma2; e3 = s2 / sigma3;
-    le1 = (l1 * s2) / sigma1; le2 = (l2 * s2) / sigma2; le3 = (l3 * s2) / sigma3;
-    ve1 = (vroe * s2) / sigma1; ve2 = (vroe * s2) / sigma2; ve3 = (vroe * s2) / sigma3;
-    ce1 = (croe * s2) / sigma1; ce2 = (croe * s2) / sigma2; ce3 = (croe * s2) / sigma3;
-  }
-  // rows 0-3 of manapy's rmat (row 4 only feeds the bed flux, identically zero)
-  const double r00 = sign1 * g1 - sign2 * g2 + sign3 * g3;
-  const double r10 = l1 * g1 - l2 * g2 + l3 * g3;
-  const double r20 = vroe * sign1 * g1 - vroe * sign2 * g2 + vroe * sign3 * g3 - vroe * sign5;
-  const double r30 = croe * sign1 * g1 - croe * sign2 * g2 + croe * sign3 * g3 - croe * sign4;
-  const double r01 = -sign1 * q1 + sign2 * q2 - sign3 * q3;
-  const double r11 = -sign1 * lq1 * sign1 + sign2 * lq2 * sign2 - sign3 * lq3 * sign3;
-  const double r21 = -sign1 * vq1 + sign2 * vq2 - sign3 * vq3;
-  const double r31 = -sign1 * cq1 + sign2 * cq2 - sign3 * cq3;
-  const double r04 = sign1 * e1 - sign2 * e2 + sign3 * e3;
-  const double r14 = le1 - le2 + le3;
-  const double r24 = sign1 * ve1 - sign2 * ve2 + sign3 * ve3;
-  const double r34 = sign1 * ce1 - sign2 * ce2 + sign3 * ce3;
-  const double hnew = r00 * wd0 + r01 * wd1 + r04 * wd4;
-  const double unew0 = r10 * wd0 + r11 * wd1 + r14 * wd4;
-  const double vnew0 = r20 * wd0 + r21 * wd1 + sign5 * wd2 + r24 * wd4;
-  const double cnew = r30 * wd0 + r31 * wd1 + sign4 * wd3 + r34 * wd4;
-  w_lrh = w_lrh - hnew / 2;
-  w_lrhu = w_lrhu - unew0 / 2;
-  w_lrhv = w_lrhv - vnew0 / 2;
-  w_lrhc = w_lrhc - cnew / 2;
-  double unew, vnew;
-  if (FAST) {
-    const double im = 1 / mesure;
-    unew = (w_lrhu * n0 + w_lrhv * -1 * n1) * im;
-    vnew = (w_lrhu * -1 * ninv0 + w_lrhv * ninv1) * im;
-  } else {
-    unew = (w_lrhu * n0 + w_lrhv * -1 * n1) / mesure;
-    vnew = (w_lrhu * -1 * ninv0 + w_lrhv * ninv1) / mesure;
-  }
+  const bool za = fabs(a) < eps, zb = fabs(b) < eps;
+  const double sa = za ? 0. : copysign(1.0, a);
+  const double sb = zb ? 0. : copysign(1.0, b);
+  const double s0 = fabs(u) < eps ? 0. : copysign(1.0, u);
+  const double da = za ? 1. : a, db = zb ? 1. : b, c2 = 2 * c;
+  const double dab = da * db;
+  const double D = 1 / (c2 * dab);
+  const double i2c = D * dab;
+  // sign(a) / a - sign(b) / b
+  const double e = (sa * db - sb * da) * (D * c2);
+  const double ds = sa - sb;
+  const double hnew = ((sb * a - sa * b) * wd0 + ds * wd1) * i2c + 0.5 * c * e * wd4;
+  const double unew0 = ((a * sa - b * sb) * wd1 - a * b * ds * wd0) * i2c + 0.5 * c * ds * wd4;
+  const double vnew0 = v * hnew + s0 * (wd2 - v * wd0);
+  const double cnew = c_h * hnew + s0 * (wd3 - c_h * wd0);
+  const double w_lrh = hroe - hnew / 2;
+  const double w_lrhu = (uleft + uright) / 2 - unew0 / 2;
+  const double w_lrhv = (vleft + vright) / 2 - vnew0 / 2;
+  const double w_lrhc = (hc_l + hc_r) / 2 - cnew / 2;
+  const double unew = w_lrhu * m0 - w_lrhv * m1;
+  const double vnew = w_lrhu * m1 + w_lrhv * m0;
   const double q_s = n0 * unew + n1 * vnew;
   const double gh = 0.5 * grav * w_lrh * w_lrh;
+  const double qw = q_s / w_lrh;
   flux[0] = q_s;
-  if (FAST) {
-    const double iw = 1 / w_lrh;
-    flux[1] = q_s * unew * iw + gh * n0;
-    flux[2] = q_s * vnew * iw + gh * n1;
-    flux[3] = q_s * w_lrhc * iw;
-  } else {
-    flux[1] = q_s * unew / w_lrh + gh * n0;
-    flux[2] = q_s * vnew / w_lrh + gh * n1;
-    flux[3] = q_s * w_lrhc / w_lrh;
-  }
+  flux[1] = qw * unew + gh * n0;
+  flux[2] = qw * vnew + gh * n1;
+  flux[3] = qw * w_lrhc;
 }
 
 struct SWState {
@@ -509,10 +424,6 @@ __global__ void __launch_bounds__(kBlock) k_sw_cell_update(mb_mesh m, SWState s,
 // step from the updated state (manapy's time_step_SW on that state), reduced
 // into dt_next.
 
-#ifndef MB_SW_FAST
-#define MB_SW_FAST 1
-#endif
-
 __device__ __forceinline__ int4 ldi4(const int32_t *p) { return __ldg(reinterpret_cast<const int4 *>(p)); }
 __device__ __forceinline__ double2 ldd2s(const double *p) { return __ldg(reinterpret_cast<const double2 *>(p)); }
 __device__ __forceinline__ int compi(const int4 v, int j) { return j == 0 ? v.x : (j == 1 ? v.y : v.z); }
@@ -528,7 +439,7 @@ __device__ __forceinline__ int compi(const int4 v, int j) { return j == 0 ? v.x 
 #endif
 
 // SRNH flux of face f of the compact-layout step, written as one 32-byte record.
-template <bool ORDER2, bool FAST>
+template <bool ORDER2>
 __device__ __forceinline__ void sw2_flux_face(const mb_mesh &m, const SWState &s, double grav, double *ff, int f) {
   const int l = ld(m.face_cellid + 2 * f), r = ld(m.face_cellid + 2 * f + 1);
   const double n0 = ld(m.face_normal + 3 * f), n1 = ld(m.face_normal + 3 * f + 1), mes = ld(m.face_mesure + f);
@@ -557,7 +468,7 @@ __device__ __forceinline__ void sw2_flux_face(const mb_mesh &m, const SWState &s
     hv_r = ld(s.q[2] + rr);
   }
   double fl[4];
-  srnh0<FAST>(hu_l, hu_r, hv_l, hv_r, h_l, h_r, hc_l, hc_r, ld(s.q[4] + l), ld(s.q[4] + rr), n0, n1, mes, grav, fl);
+  srnh0(hu_l, hu_r, hv_l, hv_r, h_l, h_r, hc_l, hc_r, ld(s.q[4] + l), ld(s.q[4] + rr), n0, n1, 1 / mes, grav, fl);
 #if MB_V4_IO
   st4d_plain(ff + 4 * (long long)f, fl[0], fl[1], fl[2], fl[3]);
 #else
@@ -566,13 +477,13 @@ __device__ __forceinline__ void sw2_flux_face(const mb_mesh &m, const SWState &s
 #endif
 }
 
-template <bool ORDER2, bool FAST>
+template <bool ORDER2>
 __global__ void __launch_bounds__(MB_SW_FLUX_BLOCK, MB_SW_FLUX_MIN_BLOCKS) k_sw2_flux(mb_mesh m, SWState s, double grav, double *ff,
                                                      double *dt_next) {
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f == 0 && dt_next) *dt_next = 1e6;
   if (f >= m.nbfaces) return;
-  sw2_flux_face<ORDER2, FAST>(m, s, grav, ff, f);
+  sw2_flux_face<ORDER2>(m, s, grav, ff, f);
 }
 
 // CFL dt candidate of a cell (manapy/solvers/shallowater/fvm_utils.py:16-42, without
@@ -581,14 +492,16 @@ __global__ void __launch_bounds__(MB_SW_FLUX_BLOCK, MB_SW_FLUX_MIN_BLOCKS) k_sw2
 // it (the fused step's next dt, mb_sw_dt) gives the same bits.
 __device__ __forceinline__ double sw_dt_candidate(double h, double hu, double hv, const double n0[3],
                                                   const double n1[3], double vol, double cfl, double grav) {
+  // manapy's (|u.n| / mesure + velson) * mesure, without the division
   const double velson = __dsqrt_rn(__dmul_rn(grav, h));
-  const double u = __ddiv_rn(hu, h), v = __ddiv_rn(hv, h);
+  const double ih = __ddiv_rn(1.0, h);
+  const double u = __dmul_rn(hu, ih), v = __dmul_rn(hv, ih);
   double lam = 0.;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
     const double mes = __dsqrt_rn(__dadd_rn(__dmul_rn(n0[j], n0[j]), __dmul_rn(n1[j], n1[j])));  // faces.mesure
     const double u_n = fabs(__dadd_rn(__dmul_rn(u, n0[j]), __dmul_rn(v, n1[j])));
-    lam = __dadd_rn(lam, __dmul_rn(__dadd_rn(__ddiv_rn(u_n, mes), velson), mes));
+    lam = __dadd_rn(lam, __dadd_rn(u_n, __dmul_rn(velson, mes)));
   }
   return __ddiv_rn(__dmul_rn(cfl, vol), lam);
 }
@@ -728,7 +641,8 @@ __device__ __forceinline__ double sw2_cell_body(const mb_mesh &m, const SWState 
                         (mata[0] * c_2 - matb[0] * c_1);
   const double deltaz = (mata[1] * c_2 - matb[1] * c_1) - (mata[0] * c_2 - matb[0] * c_1) +
                         c_3 * (mata[0] * matb[1] - matb[0] * mata[1]);
-  const double h_1 = deltax / delta, h_2 = deltay / delta, h_3 = deltaz / delta;
+  const double rdelta = 1 / delta;
+  const double h_1 = deltax * rdelta, h_2 = deltay * rdelta, h_3 = deltaz * rdelta;
   const double z_1 = Z_i + h_i - h_1, z_2 = Z_i + h_i - h_2, z_3 = Z_i + h_i - h_3;
   const double ns0x = (G.y - P1.y), ns0y = -(G.x - P1.x);
   const double ns1x = ns0x - ss0[1], ns1y = ns0y - ss1[1];
@@ -742,11 +656,11 @@ __device__ __forceinline__ double sw2_cell_body(const mb_mesh &m, const SWState 
   const double shu = -grav * (s1x + s2x + s3x);
   const double shv = -grav * (s1y + s2y + s3y);
   // update (manapy/solvers/shallowater/fvm_utils.py:3-14, no Coriolis/wind/diffusion)
-  const double dt = *dt_cur;
-  const double h_n = h_i + dt * (rez[0] + 0.) / vol;
-  const double hu_n = hu_i + dt * ((rez[1] + shu) / vol + 0. + 0.);
-  const double hv_n = hv_i + dt * ((rez[2] + shv) / vol + 0. + 0.);
-  const double hc_n = hc_i + dt * (rez[3] + 0. - 0.) / vol;
+  const double dtv = *dt_cur / vol;
+  const double h_n = h_i + dtv * rez[0];
+  const double hu_n = hu_i + dtv * (rez[1] + shu);
+  const double hv_n = hv_i + dtv * (rez[2] + shv);
+  const double hc_n = hc_i + dtv * rez[3];
   out.q[0][i] = h_n;
   out.q[1][i] = hu_n;
   out.q[2][i] = hv_n;
@@ -811,7 +725,7 @@ __global__ void __launch_bounds__(MB_SW_FLUX_BLOCK, MB_SW_FLUX_MIN_BLOCKS)
   if (f >= it.m.nbfaces) return;
   SWState s{};
   for (int k = 0; k < 5; ++k) s.q[k] = it.q[par][k];
-  sw2_flux_face<false, MB_SW_FAST>(it.m, s, it.grav, it.face_flux, f);
+  sw2_flux_face<false>(it.m, s, it.grav, it.face_flux, f);
 }
 
 #ifndef MB_SW_BATCH_CELL_MIN_BLOCKS
@@ -962,9 +876,9 @@ static int sw_step(const mb_mesh *m, const double *const q_in[5], double *const 
     if (rc != MB_OK) return rc;
     s.gr[0] = hx; s.gr[1] = hy; s.gr[2] = cx; s.gr[3] = cy;
     s.psi = psi;
-    k_sw2_flux<true, MB_SW_FAST><<<fb, MB_SW_FLUX_BLOCK, 0, st>>>(*m, s, grav, face_flux, dt_next);
+    k_sw2_flux<true><<<fb, MB_SW_FLUX_BLOCK, 0, st>>>(*m, s, grav, face_flux, dt_next);
   } else {
-    k_sw2_flux<false, MB_SW_FAST><<<fb, MB_SW_FLUX_BLOCK, 0, st>>>(*m, s, grav, face_flux, dt_next);
+    k_sw2_flux<false><<<fb, MB_SW_FLUX_BLOCK, 0, st>>>(*m, s, grav, face_flux, dt_next);
   }
   if (c1 > c0)
     k_sw2_cell<<<ceil_div(c1 - c0, kBlock), kBlock, 0, st>>>(*m, s, out, face_flux, dt_cur, dt_next, cfl, grav, c0, c1);
