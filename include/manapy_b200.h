@@ -298,6 +298,54 @@ int mb_advdiff_step(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_params *
                     const double *w_in, double *w_out, const double *sign_cf, const double *src,
                     const double *dt_dev, double *cell_scratch, double *node_scratch, void *stream);
 
+/* ---- one-launch step on tiles of cells (triangles) -------------------------------------- */
+
+/* Tiles: contiguous ranges of `cells` cells, each carried through the step by one block in
+ * shared memory.  Local cell indices of a tile: offset in the range, then cells + e for the
+ * outside cell ext[e] (the n1 cells across a face of the tile, then the other cells sharing a
+ * vertex with one of these cells + n1).  Tables of tile k start at k times their stride. */
+#define MB_TILE_MAX_CELLS 1024
+typedef struct mb_tiles {
+  int32_t cells, count;          /* cells per tile (even, 32 .. MB_TILE_MAX_CELLS), ceil(nbcells / cells) tiles */
+  int32_t face_cap, ext_cap;     /* strides: >= n1, >= outside cells */
+  int32_t node_cap, grp_cap;     /* >= local nodes, a multiple of 8; >= ceil(node_cap / 32) + 1, of 4 */
+  int32_t inc_cap, pad_;         /* >= entries of the node lists, a multiple of 32 */
+  /* every table starts on 16 bytes */
+  int32_t *head;                 /* [count][4] n1, outside cells, local nodes, list entries */
+  int32_t *ext;                  /* [count][ext_cap] outside cells */
+  double *ext_xy;                /* [count][ext_cap][2] their centres */
+  int32_t *node;                 /* [count][node_cap] vertices */
+  uint16_t *count16;             /* [count][node_cap] cells of the vertex; bit 15: it has boundary faces */
+  double *node_c, *node_mu;      /* [count][node_cap][2] mean centre of the vertex's cells, and weights mu */
+  uint16_t *cell;                /* [count][cells + face_cap][8] local vertices (3), local neighbours (3; 0xffff:
+                                    boundary face), flags: bit j faces.cellid[f][0] is the cell, bits 3+2j.. the
+                                    neighbour's local face, bit 9 the cell has stencil ghosts */
+  double *cell_q0, *cell_q1;     /* [count][cells + face_cap][2] rows of the least-squares reconstruction */
+  int32_t *grp;                  /* [count][grp_cap] offsets of the node lists of 32 nodes each */
+  uint16_t *inc;                 /* [count][inc_cap] node -> local cells, SELL-32, a list's first cell past its end */
+  double *node_kappa;            /* [nbnodes] sum of the vertex's centre -> vertex weights over its cells */
+} mb_tiles;
+
+/* Sizes of the tiles of a mesh (compact triangle tables): head [count][4]; *status (device,
+ * zero before) becomes 1 when the mesh cannot be tiled this way.  Set-up, once per mesh; no
+ * counterpart in manapy. */
+int mb_tile_sizes(const mb_mesh *m, int32_t cells, int32_t *head, int32_t *status, void *stream);
+/* Fills every table of t (t->head from mb_tile_sizes).  scratch: 4 (nbcells + nbnodes) doubles,
+ * 32-byte aligned, free after the call's work has run. */
+int mb_tile_fill(const mb_mesh *m, const mb_tiles *t, double *scratch, void *stream);
+/* Bytes of shared memory a block of the step takes with the strides of t (sizes only are read). */
+int mb_tile_bytes(const mb_tiles *t);
+/* The diffusive flux sum of every cell as a linear form, [6][nbcells]: c_1, c_2 of the vertex
+ * differences V_1 - V_0, V_2 - V_0, B_0..B_2 of the value differences across the faces,
+ * 1 / volume.  Depends on the mesh, the diffusion coefficients and bc->face_grad_on. */
+int mb_tile_coef(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_params *p, double *coef, void *stream);
+/* mb_advdiff_step (manapy/solvers/advecdiff/system.py:156-172) in one launch on the tiles of m.
+ * Equal to it up to rounding.  w_in 16-byte, sign_cf 32-byte aligned; coef from mb_tile_coef
+ * (diffusion). */
+int mb_advdiff_step_tile(const mb_mesh *m, const mb_tiles *t, const mb_bc *bc, const mb_advdiff_params *p,
+                         const double *w_in, double *w_out, const double *sign_cf, const double *coef,
+                         const double *src, const double *dt_dev, void *stream);
+
 /* Rows {centre, value} of a state, [nbcells][4] doubles, 32-byte aligned: {x, y, w, 0} for
  * triangles, {x, y, z, w} for tetrahedra (no counterpart in manapy). */
 int mb_pack_rows(const mb_mesh *m, const double *w, double *rows, void *stream);

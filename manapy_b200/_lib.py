@@ -50,6 +50,13 @@ class MbAdvDiffParams(ctypes.Structure):
     _fields_ = [("order", _i32), ("diffusion", _i32), ("Dxx", _d), ("Dyy", _d), ("Dzz", _d)]
 
 
+class MbTiles(ctypes.Structure):
+    _fields_ = [("cells", _i32), ("count", _i32), ("face_cap", _i32), ("ext_cap", _i32), ("node_cap", _i32),
+                ("grp_cap", _i32), ("inc_cap", _i32), ("pad_", _i32), ("head", _vp), ("ext", _vp), ("ext_xy", _vp),
+                ("node", _vp), ("count16", _vp), ("node_c", _vp), ("node_mu", _vp), ("cell", _vp), ("cell_q0", _vp),
+                ("cell_q1", _vp), ("grp", _vp), ("inc", _vp), ("node_kappa", _vp)]
+
+
 class MbAdvDiffItem(ctypes.Structure):
     _fields_ = [("m", MbMesh), ("bc", MbBC), ("p", MbAdvDiffParams), ("w", _vp * 2), ("lo", _vp * 2), ("sign_cf", _vp),
                 ("src", _vp), ("dt_dev", _vp), ("cell_scratch", _vp), ("node_scratch", _vp),
@@ -144,6 +151,12 @@ _SIGS = {
     "mb_euler_tables_2d": [_M, _vp, _vp, _vp],
     "mb_euler_step_2d": [_M, _P5, _P5, _d, _d, _vp, _vp, _vp, _vp, _i32, _vp, _vp],
     "mb_advdiff_step": [_M, _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
+    "mb_tile_sizes": [_M, _i32, _vp, _vp, _vp],
+    "mb_tile_fill": [_M, ctypes.POINTER(MbTiles), _vp, _vp],
+    "mb_tile_bytes": [ctypes.POINTER(MbTiles)],
+    "mb_tile_coef": [_M, _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp],
+    "mb_advdiff_step_tile": [_M, ctypes.POINTER(MbTiles), _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp, _vp,
+                             _vp, _vp, _vp],
     "mb_face_sign": [_M, _vp, _vp, _vp, _vp, _vp],
     "mb_pack_rows": [_M, _vp, _vp, _vp],
     "mb_lsq_matrix": [_M, _vp, _vp],

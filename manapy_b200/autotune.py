@@ -8,7 +8,8 @@ are bandwidth-bound and any depth is as fast.
 ``launch_variant(solver)``: the launch shape (threads per block and resident blocks
 per SM, four pre-built instantiations of each) of the two fused phases of the FP64
 second-order step with diffusion, chosen per phase: the first phase's variant with
-the second at its default, then the second phase's.
+the second at its default, then the second phase's.  The one-launch step on tiles has none
+to choose.
 
 Both tuners time the candidates on the solver's own mesh (CUDA events, after a
 warm-up replay), keep the fastest, restore the solver's state exactly, and remember
@@ -89,7 +90,7 @@ def launch_variant(solver, steps=64):
     s._setup()
     dm = s._dm
     if not (s.precision == "fp64" and s.order == 2 and s.diffusion and "cell_vtx" in dm.t) or \
-            dm.nbcells < SMALL:
+            dm.nbcells < SMALL or s._tiles is not None:
         return 0
     k = ("variant",) + _key(s)
     if k in _cache:

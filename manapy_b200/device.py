@@ -391,6 +391,76 @@ class DeviceMesh:
         self.t["cell_lsq"] = out
         self.struct.cell_lsq = out.data_ptr()
 
+    # cells of a tile of the one-launch triangle step (fv_tile.cu).  A B200 runs TILE_SLOTS blocks of
+    # that kernel at once (148 SMs x 3); TILE_CELLS is the most for which three blocks' shared
+    # memory fits an SM.  A mesh that fits one round of blocks gets tiles of one round (62,658
+    # cells: 144 cells, 7.4 us; 384 cells, 12.2 us); a larger one whole rounds of equal tiles, but
+    # not below 256 cells, where the cells around a tile cost more than a short last round (180,000
+    # cells: 256 cells, 14.0 us; 208, 15.4 us; 384, 16.5 us)
+    TILE_CELLS = 384
+    TILE_SLOTS = 444
+    # where a tile takes more shared memory than leaves room for two blocks per SM (vertices of
+    # hundreds of cells), the two-launch step is used
+    TILE_BYTES = 113 * 1024
+
+    @classmethod
+    def tile_cells(cls, nbcells):
+        nbcells = int(nbcells)
+        rounds = -(-nbcells // (cls.TILE_SLOTS * cls.TILE_CELLS))
+        per = 16 * -(-nbcells // (16 * cls.TILE_SLOTS * rounds))
+        return min(cls.TILE_CELLS, max(32 if rounds == 1 else 256, per))
+
+    def tiles(self, stream=None, cells=None):
+        """The tiles of a triangle mesh (``_lib.MbTiles``), built on the device on first use; None
+        where the one-launch step does not apply: tetrahedra, the ``"manapy"`` stencil layout
+        (whose results must not depend on the other cells' numbering), a table it reads is
+        missing, or the mesh has vertices of so many cells that its tiles do not fit."""
+        cells = self.tile_cells(self.nbcells) if cells is None else int(cells)
+        if getattr(self, "_tiles", None) is None:
+            self._tiles = {}
+        if cells not in self._tiles:
+            self._tiles[cells] = self._build_tiles(cells, stream)
+        got = self._tiles[cells]
+        return None if got is None else got[0]
+
+    def _build_tiles(self, cells, stream):
+        need = ("cell_vtx", "cell_xy", "n2c_ptr", "n2c_alpha", "n2g_ptr", "n2g_alpha", "lsq_sell_idx", "ghostnid_ptr",
+                "face_ghostcenter")
+        if self.dim != 2 or self.device is None or self.stencil != "shared" or any(n not in self.t for n in need):
+            return None
+        dev = self.device
+        st = stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
+        count = -(-self.nbcells // cells)
+        head = torch.empty(4 * count + 4, dtype=torch.int32, device=dev)
+        status = head[4 * count:]
+        status.zero_()
+        _lib.call("mb_tile_sizes", self.struct, cells, head.data_ptr(), status.data_ptr(), st)
+        n1, ext, nodes, inc, bad = torch.cat([torch.amax(head[:4 * count].view(-1, 4), 0), status[:1]]).tolist()
+        if bad:
+            return None
+        t = _lib.MbTiles()
+        t.cells, t.count = cells, count
+        up = lambda n, k: -(-n // k) * k  # noqa: E731
+        t.face_cap, t.ext_cap, t.node_cap = n1, ext, up(nodes, 8)
+        t.grp_cap, t.inc_cap = up(-(-t.node_cap // 32) + 1, 4), up(inc, 32)
+        if _lib.lib().mb_tile_bytes(t) > self.TILE_BYTES:
+            return None
+        # bytes of every table; one allocation, tables at 256-byte boundaries
+        sizes = {"ext": 4 * count * ext, "ext_xy": 16 * count * ext, "node": 4 * count * t.node_cap,
+                 "count16": 2 * count * t.node_cap, "node_c": 16 * count * t.node_cap,
+                 "node_mu": 16 * count * t.node_cap, "cell": 16 * count * (cells + n1),
+                 "cell_q0": 16 * count * (cells + n1), "cell_q1": 16 * count * (cells + n1),
+                 "grp": 4 * count * t.grp_cap, "inc": 2 * count * t.inc_cap, "node_kappa": 8 * self.nbnodes}
+        buf = torch.empty(sum(up(n, 256) for n in sizes.values()) + 256, dtype=torch.uint8, device=dev)
+        at = up(buf.data_ptr(), 256)
+        for k, n in sizes.items():
+            setattr(t, k, at)
+            at += up(n, 256)
+        t.head = head.data_ptr()
+        scratch = torch.empty(4 * (self.nbcells + self.nbnodes), dtype=torch.float64, device=dev)
+        _lib.call("mb_tile_fill", self.struct, t, scratch.data_ptr(), st)
+        return t, (head, buf)
+
     def upload(self, device, stream=None):
         """Move host-built tables (``device=None`` at construction) to ``device``; with a
         CUDA ``stream`` the copies are asynchronous on it.  Drops the host arrays ``A``."""

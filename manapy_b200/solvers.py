@@ -5,8 +5,8 @@ and ``ShallowWaterSolver`` mirrors ``manapy/solvers/shallowater/system.py:23-281
 same options, same validation errors, same ``stepper()`` /
 ``compute_fluxes()`` / ``compute_new_val()`` sequence.
 
-Execution: ``compute_new_val()`` runs one fused step (two kernel launches for
-advection-diffusion, three for shallow water) that recomputes what
+Execution: ``compute_new_val()`` runs one fused step (one kernel launch for FP64
+advection-diffusion on triangles, two or three elsewhere) that recomputes what
 ``compute_fluxes()`` would have produced on the fly.  The intermediate arrays
 manapy leaves behind (``var.ghost``, ``var.convective``, ``var.dissipative``,
 ``var.gradfacex/y/z``) are still available: reading one runs the matching
@@ -158,6 +158,13 @@ class AdvectionDiffusionSolver:
             self._sign = torch.zeros(4 * self._dm.nbcells, dtype=torch.float64, device=dev)
             self._params = _lib.MbAdvDiffParams(int(self.order), int(self.diffusion), float(self.Dxx),
                                                 float(self.Dyy), float(self.Dzz))
+            self._tiles = self._coef = None
+            if self.precision == "fp64" and self.launch == "auto" and (self.order == 2 or self.diffusion):
+                self._tiles = self._dm.tiles(self._stream())   # triangles: the one-launch step
+            if self._tiles is not None and self.diffusion:
+                self._coef = torch.empty(6 * self._dm.nbcells, dtype=torch.float64, device=dev)
+                _lib.call("mb_tile_coef", self._dm.struct, self.var.device_bc.struct, self._params, _p(self._coef),
+                          self._stream())
         return self._dm
 
     def _stream(self):
@@ -317,25 +324,34 @@ class AdvectionDiffusionSolver:
             self._rows_version = self.var.version("cell")
         return self._rows_of(buf)
 
+    def _call_step(self, w_in, w_out, src, st):
+        """The kernels of one FP64 step (the rows of ``w_in`` current where they are used)."""
+        dm, bc = self._dm, self.var.device_bc.struct
+        if self._tiles is not None:
+            _lib.call("mb_advdiff_step_tile", dm.struct, self._tiles, bc, self._params, _p(w_in), _p(w_out),
+                      _p(self._sign), _p(self._coef), src, _p(self._dt_dev), st)
+            return
+        cs, ns = self._scratch()
+        if self._use_rows():
+            _lib.call("mb_advdiff_step_rows", dm.struct, bc, self._params, _p(w_in), _p(w_out),
+                      _p(self._rows_of(w_in)), _p(self._rows_of(w_out)), _p(self._sign), src, _p(self._dt_dev),
+                      _p(cs), _p(ns), st)
+        else:
+            _lib.call("mb_advdiff_step", dm.struct, bc, self._params, _p(w_in), _p(w_out), _p(self._sign), src,
+                      _p(self._dt_dev), _p(cs), _p(ns), st)
+
     def _fused_step(self):
         if self.precision == "fp32c":
             return self._fused_step_f32c()
         var = self.var
-        dm = self._dm
         self._update_sign()
         w_in = var.dev("cell")
         if self._spare is None or self._spare.numel() != w_in.numel():
             self._spare = torch.empty_like(w_in)
         w_out = self._spare
-        cs, ns = self._scratch()
         if self._use_rows():
-            rin = self._ensure_rows(w_in)
-            _lib.call("mb_advdiff_step_rows", dm.struct, var.device_bc.struct, self._params, _p(w_in), _p(w_out),
-                      _p(rin), _p(self._rows_of(w_out)), _p(self._sign), self._source_ptr(), _p(self._dt_dev), _p(cs),
-                      _p(ns), self._stream())
-        else:
-            _lib.call("mb_advdiff_step", dm.struct, var.device_bc.struct, self._params, _p(w_in), _p(w_out),
-                      _p(self._sign), self._source_ptr(), _p(self._dt_dev), _p(cs), _p(ns), self._stream())
+            self._ensure_rows(w_in)
+        self._call_step(w_in, w_out, self._source_ptr(), self._stream())
         self._spare = var.swap_cell(w_out)
         self._install_lazies(self._spare)
         self._rows_version = var.version("cell")
@@ -426,6 +442,8 @@ class AdvectionDiffusionSolver:
         # carry them from one step to the next instead; with the edge sums the first phase is
         # two launches: vertex and edge sums, then the cells)
         dm = self._dm
+        if dm is not None and self._tiles is not None:
+            return 1
         sums = dm is not None and self.order == 2 and dm.struct is not None and bool(dm.struct.cell_edges)
         return 1 + int(self.order == 2 or bool(self.diffusion)) + int(sums)
 
@@ -532,8 +550,9 @@ class AdvectionDiffusionSolver:
         a = var.dev("cell")
         b = self._spare
         dm = self._dm
-        cs, ns = self._scratch()
-        args = (var.device_bc.struct, self._params)
+        if self._tiles is None:
+            self._scratch()             # allocated before the capture
+        var.device_bc
         src = self._source_ptr()
         s = torch.cuda.Stream(device=dm.device)
         s.wait_stream(torch.cuda.current_stream(dm.device))
@@ -546,13 +565,7 @@ class AdvectionDiffusionSolver:
             with torch.cuda.graph(g, stream=s):
                 st = torch.cuda.current_stream(dm.device).cuda_stream
                 for x, y in ((a, b), (b, a)) * (int(self.graph_depth) // 2):
-                    if rows:
-                        _lib.call("mb_advdiff_step_rows", dm.struct, args[0], args[1], _p(x), _p(y),
-                                  _p(self._rows_of(x)), _p(self._rows_of(y)), _p(self._sign), src, _p(self._dt_dev),
-                                  _p(cs), _p(ns), st)
-                    else:
-                        _lib.call("mb_advdiff_step", dm.struct, args[0], args[1], _p(x), _p(y), _p(self._sign),
-                                  src, _p(self._dt_dev), _p(cs), _p(ns), st)
+                    self._call_step(x, y, src, st)
         torch.cuda.current_stream(dm.device).wait_stream(s)
         self._graph = g
         self._graph_bufs = (a, b)
