@@ -421,6 +421,36 @@ int mb_cell_face_sign(const mb_mesh *m, const double *u_face, const double *v_fa
 int mb_face_sign(const mb_mesh *m, const double *u_face, const double *v_face,
                  const double *w_face, double *sign_face, void *stream);
 
+/* Tiles of cells with their faces, for the one-launch shallow-water step: local cells as in mb_tiles
+ * (the outside cells are those across a face of the tile only), local faces those of the tile's
+ * cells. */
+typedef struct mb_face_tiles {
+  int32_t cells, count;          /* cells per tile (even, 32 .. MB_TILE_MAX_CELLS), ceil(nbcells / cells) tiles */
+  int32_t out_cap, face_cap;     /* strides: >= outside cells; >= faces, a multiple of 4 */
+  /* every table starts on 16 bytes */
+  int32_t *head;                 /* [count][4] outside cells, faces, 0, 0 */
+  int32_t *out;                  /* [count][out_cap] outside cells */
+  uint16_t *face;                /* [count][face_cap][2] local left and right cell (0xffff: boundary face) */
+  double *face_n0, *face_n1, *face_mes;  /* [count][face_cap] faces.normal x, y and faces.mesure */
+  uint16_t *cell;                /* [count][cells][8] local faces (3), local neighbours (3; 0xffff: boundary), flags:
+                                    bit j left cell of face j, bits 3-8 cell_order, bit 9+j cells.nf is minus the
+                                    normal, bit 12 the cell has a boundary face */
+  double *cell_ns;               /* [nbcells][2] y_G - y_1, -(x_G - x_1), 1 the cell's second vertex */
+} mb_face_tiles;
+
+/* Sizes: head [count][4]; *status (device, zero before) becomes 1 when the mesh cannot be tiled this
+ * way.  Then mb_face_tile_fill fills the tables.  Set-up, once per mesh. */
+int mb_face_tile_sizes(const mb_mesh *m, int32_t cells, int32_t *head, int32_t *status, void *stream);
+int mb_face_tile_fill(const mb_mesh *m, const mb_face_tiles *t, void *stream);
+
+/* mb_sw_step_ex in one launch on the tiles of m (after the gradients' launch at second order): the same
+ * bits.  Each face of a tile is evaluated by the tile, once in shared memory.  dt_cur is read,
+ * dt_next (1e6 before) takes the min over the new state, dt_after is set to 1e6: three distinct
+ * slots, so that consecutive steps need no other launch. */
+int mb_sw_step_tile(const mb_mesh *m, const mb_face_tiles *t, const double *const q_in[5], double *const q_out[4],
+                    double cfl, double grav, int32_t order, int32_t walls, double *scratch, const double *dt_cur,
+                    double *dt_next, double *dt_after, void *stream);
+
 /* One shallow-water step (ShallowWaterSolver.compute_fluxes + compute_new_val,
  * manapy/solvers/shallowater/system.py:248-281,237-242) with Neumann ghosts on every
  * boundary face (manapy's default), in two launches: [order 2: h, hc gradients and hc

@@ -57,6 +57,11 @@ class MbTiles(ctypes.Structure):
                 ("cell_q1", _vp), ("grp", _vp), ("inc", _vp), ("node_kappa", _vp)]
 
 
+class MbFaceTiles(ctypes.Structure):
+    _fields_ = [("cells", _i32), ("count", _i32), ("out_cap", _i32), ("face_cap", _i32), ("head", _vp), ("out", _vp),
+                ("face", _vp), ("face_n0", _vp), ("face_n1", _vp), ("face_mes", _vp), ("cell", _vp), ("cell_ns", _vp)]
+
+
 class MbAdvDiffItem(ctypes.Structure):
     _fields_ = [("m", MbMesh), ("bc", MbBC), ("p", MbAdvDiffParams), ("w", _vp * 2), ("lo", _vp * 2), ("sign_cf", _vp),
                 ("src", _vp), ("dt_dev", _vp), ("cell_scratch", _vp), ("node_scratch", _vp),
@@ -153,6 +158,9 @@ _SIGS = {
     "mb_advdiff_step": [_M, _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "mb_tile_sizes": [_M, _i32, _vp, _vp, _vp],
     "mb_tile_fill": [_M, ctypes.POINTER(MbTiles), _vp, _vp],
+    "mb_face_tile_sizes": [_M, _i32, _vp, _vp, _vp],
+    "mb_face_tile_fill": [_M, ctypes.POINTER(MbFaceTiles), _vp],
+    "mb_sw_step_tile": [_M, ctypes.POINTER(MbFaceTiles), _P5, _P4, _d, _d, _i32, _i32, _vp, _vp, _vp, _vp, _vp],
     "mb_tile_bytes": [ctypes.POINTER(MbTiles)],
     "mb_tile_coef": [_M, _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp],
     "mb_advdiff_step_tile": [_M, ctypes.POINTER(MbTiles), _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp, _vp,

@@ -57,6 +57,12 @@ class ResolvedBC:
         self.cell_writes = None  # (face ids, values) written into the cell array at set-up
 
     @property
+    def all_neumann(self):
+        """Every boundary face copies its cell's value: from the sides' rules, a handful, not from the
+        rule of every face."""
+        return all(t in ("neumann", "slip") or len(f) == 0 for t, f in self.sides.values())
+
+    @property
     def has_cell_at_face(self):
         return bool(np.any(self.kind == G_CELL_AT_FACE))
 

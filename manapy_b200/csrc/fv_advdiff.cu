@@ -1310,6 +1310,78 @@ __global__ void __launch_bounds__(kBlock) k_sw_grad(mb_mesh m, const double *h, 
   }
 }
 
+// The same on the compact tables: both fields in one walk over the stencil (each neighbour's index
+// and centre read once, one matrix), four neighbours in flight, the limiter's neighbours from
+// cell_nbr and its face centres from the vertices.  45,000 triangles (B200): 11.4 -> 7.4 us.
+__global__ void __launch_bounds__(128) k_sw_grad2(mb_mesh m, const double *__restrict__ h,
+                                                  const double *__restrict__ hc, double *__restrict__ hx,
+                                                  double *__restrict__ hy, double *__restrict__ cx,
+                                                  double *__restrict__ cy, double *__restrict__ psi) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.nbcells) return;
+  const double2 c = ldd2(m.cell_xy + 2 * (long long)i);
+  const double hi = ld(h + i), ci = ld(hc + i);
+  double ixx = 0., iyy = 0., ixy = 0., jx = 0., jy = 0., kx = 0., ky = 0.;
+  auto add = [&](double2 p, double a, double b) {
+    const double dx = p.x - c.x, dy = p.y - c.y, da = a - hi, db = b - ci;
+    ixx += dx * dx; iyy += dy * dy; ixy += dx * dy;
+    jx += dx * da; jy += dy * da;
+    kx += dx * db; ky += dy * db;
+  };
+  const int sb = ld(m.lsq_sell_ptr + (i >> 5)), se = ld(m.lsq_sell_ptr + (i >> 5) + 1);
+  const int L = (se - sb) >> 5;
+  const int32_t *ix = m.lsq_sell_idx + sb + (threadIdx.x & 31);
+  for (int k = 0; k < L; k += 4) {
+    int o[4];
+    double2 p[4];
+    double a[4], b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) o[u] = k + u < L ? ld(ix + 32 * (k + u)) : -1;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      // an empty slot: the cell itself, exact zeros
+      p[u] = o[u] < 0 ? c : ldd2(m.cell_xy + 2 * (long long)o[u]);
+      a[u] = o[u] < 0 ? hi : ld(h + o[u]);
+      b[u] = o[u] < 0 ? ci : ld(hc + o[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) add(p[u], a[u], b[u]);
+  }
+  for (int k = ld(m.ghostnid_ptr + i); k < ld(m.ghostnid_ptr + i + 1); ++k) {
+    const int f = ld(m.ghostnid_idx + k), o = ld(m.face_cellid + 2 * (long long)f);   // Neumann: the face's cell
+    add(make_double2(ld(m.face_ghostcenter + 3 * (long long)f), ld(m.face_ghostcenter + 3 * (long long)f + 1)),
+        ld(h + o), ld(hc + o));
+  }
+  const double rd = 1 / (ixx * iyy - ixy * ixy);
+  hx[i] = (iyy * jx - ixy * jy) * rd;
+  hy[i] = (ixx * jy - ixy * jx) * rd;
+  const double gx = (iyy * kx - ixy * ky) * rd, gy = (ixx * ky - ixy * kx) * rd;
+  cx[i] = gx;
+  cy[i] = gy;
+  const int4 vt = ld4(m.cell_vtx + 4 * (long long)i), nb = ld4(m.cell_nbr + 4 * (long long)i);
+  const double2 P0 = ldd2(m.node_coord + 2 * (long long)vt.x), P1 = ldd2(m.node_coord + 2 * (long long)vt.y),
+                P2 = ldd2(m.node_coord + 2 * (long long)vt.z);
+  double hi_c = ci, lo_c = ci;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int o = comp(nb, j);
+    const double b = o < 0 ? ci : ld(hc + o);
+    hi_c = pmax(hi_c, b);
+    lo_c = pmin(lo_c, b);
+  }
+  double ps = 1.;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const double2 a = j == 0 ? P0 : (j == 1 ? P1 : P2), b = j == 0 ? P1 : (j == 1 ? P2 : P0);
+    const double delta = gx * (0.5 * (a.x + b.x) - c.x) + gy * (0.5 * (a.y + b.y) - c.y);
+    if (!(fabs(delta) < 1e-8)) {
+      if (delta > 0.) ps = pmin(ps, pmin(1., (hi_c - ci) / delta));
+      if (delta < 0.) ps = pmin(ps, pmin(1., (lo_c - ci) / delta));
+    }
+  }
+  psi[i] = ps;
+}
+
 // ---------------------------------------------------------------- launch helpers
 
 inline int grid_for(long long n) {
@@ -1488,7 +1560,10 @@ int launch_step(const mb_mesh &m, const mb_bc &bc, const mb_advdiff_params &p, c
 
 int sw_gradients(const mb_mesh &m, const double *h, const double *hc, double *hx, double *hy, double *cx,
                  double *cy, double *psi, cudaStream_t st) {
-  k_sw_grad<<<grid_for(m.nbcells), kBlock, 0, st>>>(m, h, hc, hx, hy, cx, cy, psi);
+  if (m.dim == 2 && compact_tables(m) && m.ghostnid_ptr && m.ghostnid_idx && m.face_ghostcenter)
+    k_sw_grad2<<<ceil_div(m.nbcells, 128), 128, 0, st>>>(m, h, hc, hx, hy, cx, cy, psi);
+  else
+    k_sw_grad<<<grid_for(m.nbcells), kBlock, 0, st>>>(m, h, hc, hx, hy, cx, cy, psi);
   return check_launch();
 }
 

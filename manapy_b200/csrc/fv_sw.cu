@@ -11,8 +11,7 @@
 // so each face flux is computed once (face kernel, one thread per face) and the
 // five residuals are gathered per cell in manapy's order (inner faces by
 // ascending id, then boundary faces by ascending id).
-#include "fv_common.cuh"
-#include "fv_compact.cuh"
+#include "fv_sw.cuh"
 
 namespace mb {
 
@@ -118,69 +117,6 @@ __device__ __forceinline__ void srnh(double hu_l, double hu_r, double hv_l, doub
   flux[4] = As * xi * n0 * unew * uv / w3 + As * xi * n1 * vnew * uv / w3;
 }
 
-// SRNH flux specialised to manapy's constant As = 0 (d = 0, beta = 0; flux[4] is identically
-// zero), with the eigenvalues of manapy's cubic lambda (lambda^2 - 2 u lambda + u^2 - c^2) in
-// closed form, a = u + c, b = u - c and 0.  Put into manapy's rows
-//   r_k = sum_k sign(lambda_k) {gamma, alpha sums, c^2} / sigma_k
-// they cancel: with l' the other two eigenvalues sigma_k = +-(lambda_k - l')(lambda_k - l''),
-// gamma_k = c^2 - u^2 + l' l'' and c^2 - u^2 = -a b, so for lambda = a, b the three quotients
-// are -b / 2c, -1 / 2c, c / 2a and a / 2c, 1 / 2c, -c / 2b; lambda = 0 has sign 0.  Rows 2
-// and 3 (tangential velocity, tracer) are v and c_h times row 0 plus the wave of speed u.
-// Results differ from manapy's by rounding only.
-//
-// The FP64 pipe bounds the face kernels (about 500 FP64 instructions per face when written
-// row by row, with 9 divisions), so quotients that share a denominator, or whose
-// denominators may be multiplied, take one division: 1 / (sl sr (sl + sr)) for the Roe means
-// (hu_l / h_l sl = hu_l / sl), 1 / (2 c a b) for 1 / 2c, 1 / a and 1 / b, 1 / w_h.
-__device__ __forceinline__ void srnh0(double hu_l, double hu_r, double hv_l, double hv_r, double h_l, double h_r,
-                                      double hc_l, double hc_r, double Z_l, double Z_r, double n0, double n1,
-                                      double im, double grav, double flux[4]) {
-  // im: 1 / mesure
-  const double sl = sqrt(h_l), sr = sqrt(h_r);
-  const double K = 1 / (sl * sr * (sl + sr));
-  const double u_h = (hu_l * sr + hu_r * sl) * K;
-  const double v_h = (hv_l * sr + hv_r * sl) * K;
-  const double c_h = (hc_l * sr + hc_r * sl) * K;
-  const double m0 = n0 * im, m1 = n1 * im;   // unit normal; the tangent is (-m1, m0)
-  const double u = u_h * m0 + v_h * m1;
-  const double v = v_h * m0 - u_h * m1;
-  const double uleft = hu_l * m0 + hv_l * m1, vleft = hv_l * m0 - hu_l * m1;
-  const double uright = hu_r * m0 + hv_r * m1, vright = hv_r * m0 - hu_r * m1;
-  const double hroe = (h_l + h_r) / 2;
-  const double wd0 = h_r - h_l, wd1 = uright - uleft, wd2 = vright - vleft, wd3 = hc_r - hc_l, wd4 = Z_r - Z_l;
-  const double c = sqrt(grav * hroe);
-  const double a = u + c, b = u - c;
-  const double eps = 1e-10;
-  const bool za = fabs(a) < eps, zb = fabs(b) < eps;
-  const double sa = za ? 0. : copysign(1.0, a);
-  const double sb = zb ? 0. : copysign(1.0, b);
-  const double s0 = fabs(u) < eps ? 0. : copysign(1.0, u);
-  const double da = za ? 1. : a, db = zb ? 1. : b, c2 = 2 * c;
-  const double dab = da * db;
-  const double D = 1 / (c2 * dab);
-  const double i2c = D * dab;
-  // sign(a) / a - sign(b) / b
-  const double e = (sa * db - sb * da) * (D * c2);
-  const double ds = sa - sb;
-  const double hnew = ((sb * a - sa * b) * wd0 + ds * wd1) * i2c + 0.5 * c * e * wd4;
-  const double unew0 = ((a * sa - b * sb) * wd1 - a * b * ds * wd0) * i2c + 0.5 * c * ds * wd4;
-  const double vnew0 = v * hnew + s0 * (wd2 - v * wd0);
-  const double cnew = c_h * hnew + s0 * (wd3 - c_h * wd0);
-  const double w_lrh = hroe - hnew / 2;
-  const double w_lrhu = (uleft + uright) / 2 - unew0 / 2;
-  const double w_lrhv = (vleft + vright) / 2 - vnew0 / 2;
-  const double w_lrhc = (hc_l + hc_r) / 2 - cnew / 2;
-  const double unew = w_lrhu * m0 - w_lrhv * m1;
-  const double vnew = w_lrhu * m1 + w_lrhv * m0;
-  const double q_s = n0 * unew + n1 * vnew;
-  const double gh = 0.5 * grav * w_lrh * w_lrh;
-  const double qw = q_s / w_lrh;
-  flux[0] = q_s;
-  flux[1] = qw * unew + gh * n0;
-  flux[2] = qw * vnew + gh * n1;
-  flux[3] = qw * w_lrhc;
-}
-
 struct SWState {
   const double *q[5];  // h, hu, hv, hc, Z (cells)
   const double *g[5];  // ghosts (faces); null -> neumann copy of the interior cell
@@ -188,14 +124,6 @@ struct SWState {
   const double *psi;   // hc's limiter (order 2)
   int walls;           // boundary faces of the fused step: MB_WALLS_NEUMANN or MB_WALLS_REFLECT
 };
-
-// Momentum of a reflective-wall ghost: the interior momentum with its normal
-// component reversed, q - 2 (q.n) n / |n|^2 (no counterpart in manapy).
-__device__ __forceinline__ void wall_mirror(double hu, double hv, double n0, double n1, double &gu, double &gv) {
-  const double k = 2 * (hu * n0 + hv * n1) / (n0 * n0 + n1 * n1);
-  gu = hu - k * n0;
-  gv = hv - k * n1;
-}
 
 __device__ __forceinline__ double sw_ghost(const SWState &s, int k, int f, int c0) {
   return s.g[k] ? ld(s.g[k] + f) : ld(s.q[k] + c0);
@@ -447,17 +375,9 @@ __device__ __forceinline__ void sw2_flux_face(const mb_mesh &m, const SWState &s
   const int rr = r >= 0 ? r : l;  // Neumann ghost: the interior cell's state
   double h_r = ld(s.q[0] + rr), hc_r = ld(s.q[3] + rr);
   if (ORDER2) {
-    const double *fc = m.face_center + 3 * f, *cc = m.cell_center;
-    const double rl0 = ld(fc) - ld(cc + 3 * l), rl1 = ld(fc + 1) - ld(cc + 3 * l + 1);
-    const double pl = ld(s.psi + l);
-    h_l = h_l + pl * (ld(s.gr[0] + l) * rl0 + ld(s.gr[1] + l) * rl1);
-    hc_l = hc_l + pl * (ld(s.gr[2] + l) * rl0 + ld(s.gr[3] + l) * rl1);
-    if (r >= 0) {
-      const double rr0 = ld(fc) - ld(cc + 3 * r), rr1 = ld(fc + 1) - ld(cc + 3 * r + 1);
-      const double pr = ld(s.psi + r);
-      h_r = h_r + pr * (ld(s.gr[0] + r) * rr0 + ld(s.gr[1] + r) * rr1);
-      hc_r = hc_r + pr * (ld(s.gr[2] + r) * rr0 + ld(s.gr[3] + r) * rr1);
-    }
+    const double fx = ld(m.face_center + 3 * f), fy = ld(m.face_center + 3 * f + 1);
+    sw_reconstruct(s.gr, s.psi, m.cell_center, l, fx, fy, h_l, hc_l);
+    if (r >= 0) sw_reconstruct(s.gr, s.psi, m.cell_center, r, fx, fy, h_r, hc_r);
   }
   const double hu_l = ld(s.q[1] + l), hv_l = ld(s.q[2] + l);
   double hu_r, hv_r;
@@ -468,7 +388,7 @@ __device__ __forceinline__ void sw2_flux_face(const mb_mesh &m, const SWState &s
     hv_r = ld(s.q[2] + rr);
   }
   double fl[4];
-  srnh0(hu_l, hu_r, hv_l, hv_r, h_l, h_r, hc_l, hc_r, ld(s.q[4] + l), ld(s.q[4] + rr), n0, n1, 1 / mes, grav, fl);
+  srnh0(hu_l, hu_r, hv_l, hv_r, h_l, h_r, hc_l, hc_r, ld(s.q[4] + l), ld(s.q[4] + rr), n0, n1, mes, grav, fl);
 #if MB_V4_IO
   st4d_plain(ff + 4 * (long long)f, fl[0], fl[1], fl[2], fl[3]);
 #else
@@ -484,26 +404,6 @@ __global__ void __launch_bounds__(MB_SW_FLUX_BLOCK, MB_SW_FLUX_MIN_BLOCKS) k_sw2
   if (f == 0 && dt_next) *dt_next = 1e6;
   if (f >= m.nbfaces) return;
   sw2_flux_face<ORDER2>(m, s, grav, ff, f);
-}
-
-// CFL dt candidate of a cell (manapy/solvers/shallowater/fvm_utils.py:16-42, without
-// diffusion) from its state and its three face normals, written with explicit
-// round-to-nearest operations: no multiply-add is contracted, so every kernel that calls
-// it (the fused step's next dt, mb_sw_dt) gives the same bits.
-__device__ __forceinline__ double sw_dt_candidate(double h, double hu, double hv, const double n0[3],
-                                                  const double n1[3], double vol, double cfl, double grav) {
-  // manapy's (|u.n| / mesure + velson) * mesure, without the division
-  const double velson = __dsqrt_rn(__dmul_rn(grav, h));
-  const double ih = __ddiv_rn(1.0, h);
-  const double u = __dmul_rn(hu, ih), v = __dmul_rn(hv, ih);
-  double lam = 0.;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const double mes = __dsqrt_rn(__dadd_rn(__dmul_rn(n0[j], n0[j]), __dmul_rn(n1[j], n1[j])));  // faces.mesure
-    const double u_n = fabs(__dadd_rn(__dmul_rn(u, n0[j]), __dmul_rn(v, n1[j])));
-    lam = __dadd_rn(lam, __dadd_rn(u_n, __dmul_rn(velson, mes)));
-  }
-  return __ddiv_rn(__dmul_rn(cfl, vol), lam);
 }
 
 // the three stored face normals of cell i (exact), from the compact 2D tables
@@ -531,7 +431,10 @@ __global__ void __launch_bounds__(kBlock) k_sw_dt(mb_mesh m, const double *h, co
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m.nbcells; i += gridDim.x * blockDim.x) {
     double n0[3], n1[3];
     sw_cell_normals(m, i, n0, n1);
-    best = pmin(best, sw_dt_candidate(ld(h + i), ld(hu + i), ld(hv + i), n0, n1, ld(m.cell_volume + i), cfl, grav));
+    double mes[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j) mes[j] = sw_measure(n0[j], n1[j]);
+    best = pmin(best, sw_dt_candidate(ld(h + i), ld(hu + i), ld(hv + i), n0, n1, mes, ld(m.cell_volume + i), cfl, grav));
   }
   best = block_min(best);
   if (threadIdx.x == 0 && best < 1e300) atomic_min_pos(dt, best);
@@ -591,76 +494,26 @@ __device__ __forceinline__ double sw2_cell_body(const mb_mesh &m, const SWState 
     n0[j] = x;
     n1[j] = y;
   }
-  // residuals: inner faces by ascending manapy face id, then boundary faces
-  double rez[4] = {0., 0., 0., 0.};
-#pragma unroll
-  for (int pass = 0; pass < 2; ++pass) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      const int sl = (code >> (2 * k)) & 3;
-      const int o = compi(nb, sl);
-      if ((o < 0) != (pass == 1)) continue;
-      const bool own = (fl >> sl) & 1u;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        const double v = sl == 0 ? F[0][c] : (sl == 1 ? F[1][c] : F[2][c]);
-        rez[c] = own ? rez[c] - v : rez[c] + v;
-      }
-    }
-  }
-  // bathymetry source (manapy/solvers/shallowater/fvm_utils.py:72-148)
-  double c_1 = 0., c_2 = 0., ss0[3], ss1[3], mata[3], matb[3], zv[3];
+  SwCell c;
+  c.h = h_i; c.hu = hu_i; c.hv = hv_i; c.hc = hc_i; c.Z = Z_i;
+  c.vol = vol;
+  c.ns0x = __dsub_rn(G.y, P1.y);
+  c.ns0y = -__dsub_rn(G.x, P1.x);
+  c.code = code;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
+    c.own[j] = (fl >> j) & 1u;
+    c.inner[j] = compi(nb, j) >= 0;
     const bool neg = (fl >> (9 + j)) & 1u;
-    ss0[j] = neg ? -1.0 * n0[j] : n0[j];
-    ss1[j] = neg ? -1.0 * n1[j] : n1[j];
-    double h_p1, z_p1;
-    if (compi(nb, j) >= 0) {
-      // cells.cellfid slot j (compacted; its padding already maps to manapy's wrapped last cell)
-      const int c = compi(fid, j);
-      h_p1 = ld(s.q[0] + c);
-      z_p1 = ld(s.q[4] + c);
-    } else {
-      h_p1 = h_i;  // Neumann ghost
-      z_p1 = Z_i;
-    }
-    zv[j] = z_p1;
-    mata[j] = h_p1 * ss0[j];
-    matb[j] = h_p1 * ss1[j];
-    const double hm = 0.5 * (h_i + h_p1);
-    c_1 = c_1 + (hm * 0.5 * (h_i + h_p1)) * ss0[j];
-    c_2 = c_2 + (hm * 0.5 * (h_i + h_p1)) * ss1[j];
+    c.s0[j] = neg ? -1.0 * n0[j] : n0[j];
+    c.s1[j] = neg ? -1.0 * n1[j] : n1[j];
+    // cells.cellfid slot j (compacted; its padding already maps to manapy's wrapped last cell)
+    const int o = compi(fid, j);
+    c.hp[j] = c.inner[j] ? ld(s.q[0] + o) : h_i;   // Neumann ghost
+    c.zp[j] = c.inner[j] ? ld(s.q[4] + o) : Z_i;
   }
-  const double c_3 = 3.0 * h_i;
-  const double delta = (mata[1] * matb[2] - mata[2] * matb[1]) - (mata[0] * matb[2] - matb[0] * mata[2]) +
-                       (mata[0] * matb[1] - matb[0] * mata[1]);
-  const double deltax = c_3 * (mata[1] * matb[2] - mata[2] * matb[1]) - (c_1 * matb[2] - c_2 * mata[2]) +
-                        (c_1 * matb[1] - c_2 * mata[1]);
-  const double deltay = (c_1 * matb[2] - c_2 * mata[2]) - c_3 * (mata[0] * matb[2] - matb[0] * mata[2]) +
-                        (mata[0] * c_2 - matb[0] * c_1);
-  const double deltaz = (mata[1] * c_2 - matb[1] * c_1) - (mata[0] * c_2 - matb[0] * c_1) +
-                        c_3 * (mata[0] * matb[1] - matb[0] * mata[1]);
-  const double rdelta = 1 / delta;
-  const double h_1 = deltax * rdelta, h_2 = deltay * rdelta, h_3 = deltaz * rdelta;
-  const double z_1 = Z_i + h_i - h_1, z_2 = Z_i + h_i - h_2, z_3 = Z_i + h_i - h_3;
-  const double ns0x = (G.y - P1.y), ns0y = -(G.x - P1.x);
-  const double ns1x = ns0x - ss0[1], ns1y = ns0y - ss1[1];
-  const double ns2x = ns0x + ss0[0], ns2y = ns0y + ss1[0];
-  const double s1x = 0.5 * h_1 * (zv[0] * ss0[0] + z_2 * ns0x + z_3 * (-1) * ns2x);
-  const double s1y = 0.5 * h_1 * (zv[0] * ss1[0] + z_2 * ns0y + z_3 * (-1) * ns2y);
-  const double s2x = 0.5 * h_2 * (zv[1] * ss0[1] + z_1 * (-1) * ns0x + z_3 * ns1x);
-  const double s2y = 0.5 * h_2 * (zv[1] * ss1[1] + z_1 * (-1) * ns0y + z_3 * ns1y);
-  const double s3x = 0.5 * h_3 * (zv[2] * ss0[2] + z_1 * ns2x + z_2 * (-1) * ns1x);
-  const double s3y = 0.5 * h_3 * (zv[2] * ss1[2] + z_1 * ns2y + z_2 * (-1) * ns1y);
-  const double shu = -grav * (s1x + s2x + s3x);
-  const double shv = -grav * (s1y + s2y + s3y);
-  // update (manapy/solvers/shallowater/fvm_utils.py:3-14, no Coriolis/wind/diffusion)
-  const double dtv = *dt_cur / vol;
-  const double h_n = h_i + dtv * rez[0];
-  const double hu_n = hu_i + dtv * (rez[1] + shu);
-  const double hv_n = hv_i + dtv * (rez[2] + shv);
-  const double hc_n = hc_i + dtv * rez[3];
+  double h_n, hu_n, hv_n, hc_n;
+  sw_update_cell(c, F, *dt_cur, grav, h_n, hu_n, hv_n, hc_n);
   out.q[0][i] = h_n;
   out.q[1][i] = hu_n;
   out.q[2][i] = hv_n;
@@ -668,7 +521,10 @@ __device__ __forceinline__ double sw2_cell_body(const mb_mesh &m, const SWState 
   if (out.q[4] != s.q[4]) out.q[4][i] = Z_i;  // the bed does not move
   // next step's dt from the updated state (manapy/solvers/shallowater/fvm_utils.py:16-42)
   if (!want_dt) return 1e300;
-  return sw_dt_candidate(h_n, hu_n, hv_n, n0, n1, vol, cfl, grav);
+  double mes[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) mes[j] = sw_measure(n0[j], n1[j]);
+  return sw_dt_candidate(h_n, hu_n, hv_n, n0, n1, mes, vol, cfl, grav);
 }
 
 __global__ void __launch_bounds__(kBlock) k_srnh_batch(int n, const double *st, const double *nrm,

@@ -83,6 +83,16 @@ inline bool tiles_ok(const mb_mesh *m, const mb_tiles *t) {
   return true;
 }
 
+inline bool face_tiles_ok(const mb_mesh *m, const mb_face_tiles *t) {
+  if (!t || t->cells < 32 || (t->cells & 1) || t->cells > MB_TILE_MAX_CELLS ||
+      t->count != ceil_div(m->nbcells, t->cells) || t->out_cap < 0 || t->face_cap < 4 || (t->face_cap & 3))
+    return false;
+  const void *p[] = {t->head, t->out, t->face, t->face_n0, t->face_n1, t->face_mes, t->cell, t->cell_ns};
+  for (const void *q : p)
+    if (!q || ((uintptr_t)q & 15)) return false;
+  return true;
+}
+
 // programmatic dependent launch: a step's blocks may start while the previous step's last ones
 // run; before tile_after_previous() they touch only tables that no step writes
 __device__ __forceinline__ void tile_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -106,6 +116,10 @@ inline cudaError_t tile_launch(void (*k)(P...), int blocks, int threads, int byt
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
+
+// flags of a cell record of the tiles with faces: bit j left cell of face j, bits 3-8 manapy's order of
+// the faces (cell_order), bit 9+j cells.nf is minus the face normal, and
+constexpr unsigned kTileRim = 1u << 12;     // the cell has a boundary face
 
 struct TileCell {
   int v[3], n[3];

@@ -331,6 +331,126 @@ __global__ void __launch_bounds__(kBlock) k_tile_coef(mb_mesh m, mb_bc bc, mb_ad
   out[5 * n + i] = 1 / ld(m.cell_volume + i);
 }
 
+// ---------------------------------------------------------------- tiles with their faces
+//
+// For the steps that exchange fluxes (shallow water, Euler): a tile's local cells are its own and,
+// at cells + e, the cells across its outer faces; its local faces those of its cells, in the
+// order of their first cell in the tile.
+
+struct FaceTileShared {
+  int ckey[kHashNodes];
+  uint16_t cval[kHashNodes];
+  int out[kMaxOut];
+  int base[MB_TILE_MAX_CELLS];   // faces of the tile's cells before each cell
+  int n1, bad;
+};
+
+template <bool WRITE>
+__global__ void __launch_bounds__(kTileThreads) k_face_plan(mb_mesh m, mb_face_tiles t, int32_t *head,
+                                                            int32_t *status) {
+  extern __shared__ unsigned char raw[];
+  FaceTileShared &s = *reinterpret_cast<FaceTileShared *>(raw);
+  const int T = t.cells, c0 = blockIdx.x * T, tid = threadIdx.x, nt = blockDim.x;
+  const int nc = min(T, m.nbcells - c0);
+  for (int i = tid; i < kHashNodes; i += nt) s.ckey[i] = -1;
+  if (tid == 0) s.n1 = s.bad = 0;
+  __syncthreads();
+  auto inside = [&](int c) { return c >= c0 && c < c0 + nc; };
+  // a face is listed by its first cell in the tile; two cells sharing two faces are refused (the
+  // search for a face in its neighbour would find the other one)
+  for (int k = tid; k < nc; k += nt) {
+    const int i = c0 + k;
+    const int4 nb = ld4(m.cell_nbr + 4 * (long long)i);
+    int mine = 0;
+    for (int j = 0; j < 3; ++j) {
+      const int o = comp(nb, j);
+      for (int q = 0; q < j; ++q)
+        if (o >= 0 && comp(nb, q) == o) s.bad = 1;
+      if (o < 0 || !inside(o) || o > i) ++mine;
+      if (o >= 0 && !inside(o)) {
+        bool was_new;
+        if (hash_put(s.ckey, kHashNodes, o, was_new) < 0) s.bad = 1;
+        if (was_new) {
+          const int at = atomicAdd(&s.n1, 1);
+          if (at < kMaxOut) s.out[at] = o; else s.bad = 1;
+        }
+      }
+    }
+    s.base[k] = mine;
+  }
+  __syncthreads();
+  const int n1 = min(s.n1, kMaxOut);
+  block_sort(s.out, n1);
+  __shared__ int nfaces;
+  if (tid == 0) {
+    int sum = 0;
+    for (int k = 0; k < nc; ++k) { const int x = s.base[k]; s.base[k] = sum; sum += x; }
+    nfaces = sum;
+    if (T + n1 >= kNoCell) s.bad = 1;
+    if (!WRITE) {
+      head[4 * blockIdx.x] = n1;
+      head[4 * blockIdx.x + 1] = sum;
+      head[4 * blockIdx.x + 2] = head[4 * blockIdx.x + 3] = 0;
+      if (s.bad) atomicMax(status, 1);
+    }
+  }
+  if (!WRITE) return;
+  __syncthreads();
+  if (s.bad || n1 > t.out_cap || nfaces > t.face_cap) return;
+  for (int k = tid; k < n1; k += nt) {
+    bool was_new;
+    s.cval[hash_put(s.ckey, kHashNodes, s.out[k], was_new)] = (uint16_t)(T + k);
+    t.out[(long long)blockIdx.x * t.out_cap + k] = s.out[k];
+  }
+  __syncthreads();
+  // local index of local face j of tile cell i
+  auto face_of = [&](int i, int j) {
+    const int4 nb = ld4(m.cell_nbr + 4 * (long long)i);
+    int at = s.base[i - c0];
+    for (int q = 0; q < j; ++q) {
+      const int o = comp(nb, q);
+      if (o < 0 || !inside(o) || o > i) ++at;
+    }
+    return at;
+  };
+  for (int k = tid; k < nc; k += nt) {
+    const int i = c0 + k;
+    const int4 nb = ld4(m.cell_nbr + 4 * (long long)i);
+    const uint32_t f = ld(m.cell_flags + i);
+    unsigned fl = (f & 7u) | ((unsigned)ld(m.cell_order + i) << 3) | (((f >> 9) & 7u) << 9);
+    int face[3], n[3];
+    for (int j = 0; j < 3; ++j) {
+      const int o = comp(nb, j);
+      n[j] = o < 0 ? kNoCell : (inside(o) ? o - c0 : (int)hash_get(s.ckey, s.cval, kHashNodes, o));
+      if (o < 0) fl |= kTileRim;
+      if (o >= 0 && inside(o) && o < i) {
+        const int4 back = ld4(m.cell_nbr + 4 * (long long)o);
+        face[j] = face_of(o, back.x == i ? 0 : (back.y == i ? 1 : 2));
+      } else {
+        face[j] = face_of(i, j);
+        // this cell lists the face: its cells (left first) and geometry
+        const bool left = (f >> j) & 1u;
+        const int g = ld(m.cell_faces + 4 * (long long)i + j);
+        const long long at = (long long)blockIdx.x * t.face_cap + face[j];
+        reinterpret_cast<uint32_t *>(t.face)[at] =
+            (unsigned)(left ? k : n[j]) | ((unsigned)(left ? n[j] : k) << 16);
+        t.face_n0[at] = ld(m.face_normal + 3 * (long long)g);
+        t.face_n1[at] = ld(m.face_normal + 3 * (long long)g + 1);
+        t.face_mes[at] = ld(m.face_mesure + g);
+      }
+    }
+    uint4 u;
+    u.x = (unsigned)face[0] | ((unsigned)face[1] << 16);
+    u.y = (unsigned)face[2] | ((unsigned)n[0] << 16);
+    u.z = (unsigned)n[1] | ((unsigned)n[2] << 16);
+    u.w = fl;
+    reinterpret_cast<uint4 *>(t.cell)[(long long)blockIdx.x * T + k] = u;
+    const int4 vt = ld4(m.cell_vtx + 4 * (long long)i);
+    const double2 P1 = ldd2(m.node_coord + 2 * (long long)vt.y), G = ldd2(m.cell_xy + 2 * (long long)i);
+    reinterpret_cast<double2 *>(t.cell_ns)[i] = make_double2(__dsub_rn(G.y, P1.y), -__dsub_rn(G.x, P1.x));
+  }
+}
+
 }  // namespace mb
 
 using namespace mb;
@@ -385,6 +505,39 @@ int mb_tile_coef(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_params *p, 
   MB_NVTX();
   if (tile_mesh_bad(m) || !bc || !bc->face_grad_on || !p || !coef ) return MB_EINVAL;
   k_tile_coef<<<ceil_div(m->nbcells, kBlock), kBlock, 0, ST(stream)>>>(*m, *bc, *p, coef);
+  return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
+}
+
+}  // extern "C"
+
+template <bool WRITE>
+static int run_face_plan(const mb_mesh *m, const mb_face_tiles *t, int32_t *head, int32_t *status, cudaStream_t st) {
+  k_face_plan<WRITE><<<t->count, kTileThreads, sizeof(FaceTileShared), st>>>(*m, *t, head, status);
+  return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
+}
+
+static bool face_mesh_bad(const mb_mesh *m) {
+  return !m || m->dim != 2 || m->nlf != 3 || m->nbcells <= 0 || !m->cell_vtx || !m->cell_nbr || !m->cell_flags ||
+         !m->cell_order || !m->cell_faces || !m->node_coord || !m->cell_xy || !m->face_normal || !m->face_mesure;
+}
+
+extern "C" {
+
+int mb_face_tile_sizes(const mb_mesh *m, int32_t cells, int32_t *head, int32_t *status, void *stream) {
+  MB_NVTX();
+  if (face_mesh_bad(m) || cells < 32 || (cells & 1) || cells > MB_TILE_MAX_CELLS || !head || !status) return MB_EINVAL;
+  mb_face_tiles t{};
+  t.cells = cells;
+  t.count = ceil_div(m->nbcells, cells);
+  return run_face_plan<false>(m, &t, head, status, ST(stream));
+}
+
+int mb_face_tile_fill(const mb_mesh *m, const mb_face_tiles *t, void *stream) {
+  MB_NVTX();
+  if (face_mesh_bad(m) || !face_tiles_ok(m, t)) return MB_EINVAL;
+  const int rc = run_face_plan<true>(m, t, nullptr, nullptr, ST(stream));
+  if (rc != MB_OK) return rc;
+  k_tile_filled<<<1, 32, 0, ST(stream)>>>();
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
 }
 

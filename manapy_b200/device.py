@@ -445,21 +445,75 @@ class DeviceMesh:
         t.grp_cap, t.inc_cap = up(-(-t.node_cap // 32) + 1, 4), up(inc, 32)
         if _lib.lib().mb_tile_bytes(t) > self.TILE_BYTES:
             return None
-        # bytes of every table; one allocation, tables at 256-byte boundaries
+        # bytes of every table
         sizes = {"ext": 4 * count * ext, "ext_xy": 16 * count * ext, "node": 4 * count * t.node_cap,
                  "count16": 2 * count * t.node_cap, "node_c": 16 * count * t.node_cap,
                  "node_mu": 16 * count * t.node_cap, "cell": 16 * count * (cells + n1),
                  "cell_q0": 16 * count * (cells + n1), "cell_q1": 16 * count * (cells + n1),
                  "grp": 4 * count * t.grp_cap, "inc": 2 * count * t.inc_cap, "node_kappa": 8 * self.nbnodes}
-        buf = torch.empty(sum(up(n, 256) for n in sizes.values()) + 256, dtype=torch.uint8, device=dev)
-        at = up(buf.data_ptr(), 256)
-        for k, n in sizes.items():
-            setattr(t, k, at)
-            at += up(n, 256)
-        t.head = head.data_ptr()
+        buf = self._carve(t, sizes, head)
         scratch = torch.empty(4 * (self.nbcells + self.nbnodes), dtype=torch.float64, device=dev)
         _lib.call("mb_tile_fill", self.struct, t, scratch.data_ptr(), st)
         return t, (head, buf)
+
+    def face_tiles(self, stream=None, cells=None):
+        """The tiles of a triangle mesh with their faces (``_lib.MbFaceTiles``), built on the device on
+        first use; None where the one-launch shallow-water step does not apply (a table it reads
+        is missing, or the mesh does not fit its tiles)."""
+        cells = self.face_tile_cells(self.nbcells) if cells is None else int(cells)
+        if getattr(self, "_face_tiles", None) is None:
+            self._face_tiles = {}
+        if cells not in self._face_tiles:
+            self._face_tiles[cells] = self._build_face_tiles(cells, stream)
+        got = self._face_tiles[cells]
+        return None if got is None else got[0]
+
+    # a B200 runs 148 SMs x 5 blocks of that kernel at once; with larger tiles fewer blocks fit an
+    # SM's shared memory (1.28M cells: 256 cells 80 us, 288 93).  One round of blocks where the mesh
+    # allows (45,000 cells: 64 cells 5.8 us, 112 7.3, 256 11.3), else whole rounds
+    FACE_TILE_CELLS = 256
+    FACE_TILE_SLOTS = 740
+
+    @classmethod
+    def face_tile_cells(cls, nbcells):
+        nbcells = int(nbcells)
+        rounds = -(-nbcells // (cls.FACE_TILE_SLOTS * cls.FACE_TILE_CELLS))
+        return min(cls.FACE_TILE_CELLS, max(32, 16 * -(-nbcells // (16 * cls.FACE_TILE_SLOTS * rounds))))
+
+    def _build_face_tiles(self, cells, stream):
+        need = ("cell_vtx", "cell_xy", "cell_faces", "face_normal", "face_mesure", "cell_cellfid", "face_center",
+                "cell_center")
+        if self.dim != 2 or self.device is None or any(n not in self.t for n in need):
+            return None
+        dev = self.device
+        st = stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
+        count = -(-self.nbcells // cells)
+        head = torch.empty(4 * count + 4, dtype=torch.int32, device=dev)
+        status = head[4 * count:]
+        status.zero_()
+        _lib.call("mb_face_tile_sizes", self.struct, cells, head.data_ptr(), status.data_ptr(), st)
+        out, faces, _, _, bad = torch.cat([torch.amax(head[:4 * count].view(-1, 4), 0), status[:1]]).tolist()
+        if bad:
+            return None
+        up = lambda n, k: -(-n // k) * k  # noqa: E731
+        t = _lib.MbFaceTiles()
+        t.cells, t.count, t.out_cap, t.face_cap = cells, count, out, up(faces, 4)
+        return t, (head, self._carve(t, {"out": 4 * count * out, "face": 4 * count * t.face_cap,
+                                         "face_n0": 8 * count * t.face_cap, "face_n1": 8 * count * t.face_cap,
+                                         "face_mes": 8 * count * t.face_cap, "cell": 16 * count * cells,
+                                         "cell_ns": 16 * self.nbcells}, head),
+                   _lib.call("mb_face_tile_fill", self.struct, t, st))
+
+    def _carve(self, t, sizes, head):
+        """One device allocation for the tables of ``t`` (bytes by field), at 256-byte boundaries."""
+        up = lambda n: -(-n // 256) * 256  # noqa: E731
+        buf = torch.empty(sum(up(n) for n in sizes.values()) + 256, dtype=torch.uint8, device=self.device)
+        at = up(buf.data_ptr())
+        for k, n in sizes.items():
+            setattr(t, k, at)
+            at += up(n)
+        t.head = head.data_ptr()
+        return buf
 
     def upload(self, device, stream=None):
         """Move host-built tables (``device=None`` at construction) to ``device``; with a

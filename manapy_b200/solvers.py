@@ -35,6 +35,50 @@ def _p(t):
     return t.data_ptr() if t is not None else None
 
 
+class _Graphs:
+    """Captured CUDA graphs of a solver by key, the last few used."""
+    MOST = 6
+
+    def __init__(self):
+        self.by_key = {}
+        self.seen = []
+
+    def clear(self):
+        self.by_key.clear()
+        self.seen.clear()
+
+    def get(self, key):
+        g = self.by_key.pop(key, None)
+        if g is not None:
+            self.by_key[key] = g        # most recently used last
+        return g
+
+    def worth(self, key):
+        """Whether a run of this key was asked for before: a capture costs about what launching its
+        steps one by one does, so a length seen once is not captured."""
+        if key in self.seen:
+            return True
+        self.seen = (self.seen + [key])[-2 * self.MOST:]
+        return False
+
+    def capture(self, key, device, body):
+        s = torch.cuda.Stream(device=device)
+        cur = torch.cuda.current_stream(device)
+        s.wait_stream(cur)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.stream(s):
+            g.capture_begin()
+            try:
+                body()
+            finally:
+                g.capture_end()
+        cur.wait_stream(s)
+        self.by_key[key] = g
+        while len(self.by_key) > self.MOST:
+            self.by_key.pop(next(iter(self.by_key)))
+        return g
+
+
 def check_state(arrays, nonneg=(), names=None):
     """Raise ``FloatingPointError`` if a device array holds NaN or infinity, ``ValueError``
     if an array listed in ``nonneg`` (by position) holds a negative value (the statuses
@@ -132,7 +176,8 @@ class AdvectionDiffusionSolver:
         self._sign_key = None
         self._pending = False
         self._spare = None
-        self._graph = None
+        self._graphs = _Graphs()
+        self._graph_bufs = None
         self._dt_host = None
         self._w32 = None       # FP32 ping-pong state of the fp32c mode
         self._w32_i = 0
@@ -141,7 +186,6 @@ class AdvectionDiffusionSolver:
         self._sign32_key = None
         self._src32 = None
         self._src32_key = None
-        self._graph_src = None
 
     # ------------------------------------------------------------ device helpers
     def _setup(self):
@@ -448,7 +492,8 @@ class AdvectionDiffusionSolver:
         return 1 + int(self.order == 2 or bool(self.diffusion)) + int(sums)
 
     def release_graphs(self):
-        self._graph = None
+        self._graphs.clear()
+        self._graph_bufs = None
 
     # ------------------------------------------------------------ device loop
     def advance(self, nsteps, graph=False):
@@ -469,66 +514,67 @@ class AdvectionDiffusionSolver:
         var.dev("cell")
         if self._spare is None:
             self._spare = torch.empty_like(var.dev("cell"))
-        depth = self._depth() if graph else 2
-        if not graph or n < depth:
-            for _ in range(n):
-                self._fused_step()
-        else:
-            g = self._get_graph()
-            a, b = self._graph_bufs
-            cur = var.dev("cell")
-            if cur is b:      # after an odd number of steps: one step brings the state back to a
-                self._fused_step()
+        total = n
+        if graph:
+            a = self._graph_bufs[0] if self._graph_bufs else var.dev("cell")
+            if n and self._graph_bufs and var.dev("cell") is self._graph_bufs[1]:
+                self._fused_step()      # after an odd number of steps: one brings the state back to a
                 n -= 1
-            elif cur is not a:  # a cell array installed since the capture
-                a.copy_(cur)
-                var.swap_cell(a)
-                self._spare = b
-            if self._use_rows() and n // depth:
-                self._ensure_rows(a)         # the captured steps start from a's rows
-            for _ in range(n // depth):
+            depth = self._depth()
+            for steps in self._graph_runs(n, depth):
+                g = self._get_graph(steps, depth)
+                if g is None:
+                    break
+                a = self._graph_bufs[0]
+                cur = var.dev("cell")
+                if cur is not a:        # a cell array installed since the capture
+                    a.copy_(cur)
+                    var.swap_cell(a)
+                    self._spare = self._graph_bufs[1]
+                if self._use_rows():
+                    self._ensure_rows(a)         # the captured steps start from a's rows
                 g.replay()
-            if n // depth:
+                n -= steps
                 var._s.version["cell"] += 1
                 self._install_lazies(self._spare)
                 self._rows_version = var.version("cell")
-            for _ in range(n % depth):
-                self._fused_step()
+        for _ in range(n):
+            self._fused_step()
+        n = total
         if self._dt_host is None:
             self._dt_host = float(self._dt_dev.item())
         self.dt = np.float64(self._dt_host)
         return n * self._dt_host
 
     def _advance_f32c(self, n, graph):
-        depth = self._depth() if graph else 2
-        if not graph or n < depth:
-            for _ in range(n):
+        if graph and n:
+            depth = self._depth()
+            self._f32_state()
+            if self._w32_i != 0:  # the captured steps start from buffer 0
                 self._fused_step_f32c()
-            return
-        self._f32_state()
-        if self._w32_i != 0:  # the captured pair starts from buffer 0
+                n -= 1
+            src = self._f32_inputs()
+            self.var.device_bc  # built (and uploaded) before any capture
+            for steps in self._graph_runs(n, depth):
+                key = (steps, _p(src))
+                g = self._graphs.get(key)
+                if g is None and (steps == depth or self._graphs.worth(key)):
+                    def body():
+                        for k in range(steps):
+                            self._call_f32c(k % 2, src, self._stream())
+                    g = self._graphs.capture(key, self._dm.device, body)
+                if g is None:
+                    break
+                g.replay()
+                n -= steps
+                self._f32_publish(1)
+        for _ in range(n):
             self._fused_step_f32c()
-            n -= 1
-        src = self._f32_inputs()
-        self.var.device_bc  # built (and uploaded) before any capture
-        if self._graph is None or self._graph_src != _p(src):
-            s = torch.cuda.Stream(device=self._dm.device)
-            s.wait_stream(torch.cuda.current_stream(self._dm.device))
-            g = torch.cuda.CUDAGraph()
-            with torch.cuda.stream(s):
-                with torch.cuda.graph(g, stream=s):
-                    st = torch.cuda.current_stream(self._dm.device).cuda_stream
-                    for _ in range(depth // 2):
-                        self._call_f32c(0, src, st)
-                        self._call_f32c(1, src, st)
-            torch.cuda.current_stream(self._dm.device).wait_stream(s)
-            self._graph, self._graph_src = g, _p(src)
-        for _ in range(n // depth):
-            self._graph.replay()
-        if n // depth:
-            self._f32_publish(1)
-        for _ in range(n % depth):
-            self._fused_step_f32c()
+
+    @staticmethod
+    def _graph_runs(n, depth):
+        """Lengths of the graph replays of ``n`` steps: whole graphs of ``depth``, then the even rest."""
+        return [depth] * (n // depth) + ([n % depth & ~1] if n % depth > 1 else [])
 
     def _depth(self):
         """Steps per graph replay (measured once per mesh size and scheme when 'auto'); with
@@ -541,35 +587,28 @@ class AdvectionDiffusionSolver:
             self.launch_variant = autotune.launch_variant(self)
         return int(self.graph_depth)
 
-    def _get_graph(self):
-        """``graph_depth`` fused steps (A->B, B->A, ...) captured once; the cell buffer ends
-        where it began."""
-        if self._graph is not None:
-            return self._graph
+    def _get_graph(self, steps, depth):
+        """``steps`` fused steps (A->B, B->A, ...; an even number: the state ends in the buffer where it
+        began) as a graph; None for a length other than ``depth`` on its first use."""
+        src = self._source_ptr()
+        key = (steps, src)
+        g = self._graphs.get(key)
+        if g is not None or (steps != depth and not self._graphs.worth(key)):
+            return g
         var = self.var
-        a = var.dev("cell")
-        b = self._spare
-        dm = self._dm
+        if self._graph_bufs is None:
+            self._graph_bufs = (var.dev("cell"), self._spare)
+        a, b = self._graph_bufs
         if self._tiles is None:
             self._scratch()             # allocated before the capture
+        if self._use_rows():
+            self._rows_of(a), self._rows_of(b)
         var.device_bc
-        src = self._source_ptr()
-        s = torch.cuda.Stream(device=dm.device)
-        s.wait_stream(torch.cuda.current_stream(dm.device))
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(s):
-            # warm-up outside capture is not needed: the library performs no lazy init
-            rows = self._use_rows()
-            if rows:
-                self._rows_of(a), self._rows_of(b)   # allocated before the capture
-            with torch.cuda.graph(g, stream=s):
-                st = torch.cuda.current_stream(dm.device).cuda_stream
-                for x, y in ((a, b), (b, a)) * (int(self.graph_depth) // 2):
-                    self._call_step(x, y, src, st)
-        torch.cuda.current_stream(dm.device).wait_stream(s)
-        self._graph = g
-        self._graph_bufs = (a, b)
-        return g
+
+        def body():
+            for x, y in ((a, b), (b, a)) * (steps // 2):
+                self._call_step(x, y, src, self._stream())
+        return self._graphs.capture(key, self._dm.device, body)
 
 
 class AdvectionSolver(AdvectionDiffusionSolver):
@@ -680,7 +719,10 @@ class ShallowWaterSolver:
         self.backend = self.domain.backend
         self.signature = self.domain.signature
         self._dm = None
+        self._tiles = None
         self._ff = None
+        self._ff_step = None   # (cfl, grav) of the last one-launch step, whose face fluxes are not kept
+        self._graphs = _Graphs()
         self._spare = None
         self._scratch = None
         self._dt_host = None
@@ -690,11 +732,12 @@ class ShallowWaterSolver:
         if self._dm is None:
             self._dm = self.domain.device_mesh
             dev = self._dm.device
-            # dt double buffer: slot _cur holds the dt of the current state when _dt_key matches
-            self._dt_buf = torch.zeros(2, dtype=torch.float64, device=dev)
+            # dt ring: slot _cur holds the dt of the current state when _dt_key matches; the one-launch
+            # step mins the next one into the slot after it (1e6 before) and resets the one after that
+            self._dt_buf = torch.full((4,), 1e6, dtype=torch.float64, device=dev)
             self._cur = 0
             self._dt_key = None
-            self._ff = torch.zeros(5 * self._dm.nbfaces, dtype=torch.float64, device=dev)
+            self._tiles = self._dm.face_tiles(self._stream()) if self.precision == "fp64" else None
             if self.order == 2:
                 self._scratch = torch.zeros(5 * self._dm.nbcells, dtype=torch.float64, device=dev)
         return self._dm
@@ -702,13 +745,19 @@ class ShallowWaterSolver:
     def _stream(self):
         return torch.cuda.current_stream(self._dm.device).cuda_stream
 
+    def _face_flux(self):
+        """Face fluxes of the two-launch step and scratch of the unfused kernels, on first use."""
+        if self._ff is None:
+            self._ff = torch.zeros(5 * self._dm.nbfaces, dtype=torch.float64, device=self._dm.device)
+        return self._ff
+
+    def _slot(self, k=0):
+        """dt ring slot ``k`` after the current one."""
+        at = (self._cur + k) % 4
+        return self._dt_buf[at:at + 1]
+
     def _all_neumann(self):
-        from . import boundary as B
-        for var in self.varbs.values():
-            k = var.resolved_bc.kind
-            if np.any((k != B.G_NEUMANN) & (k != B.G_NONE)):
-                return False
-        return True
+        return all(var.resolved_bc.all_neumann for var in self.varbs.values())
 
     def _q(self):
         return [self.varbs[k].dev("cell") for k in ("h", "hu", "hv", "hc", "Z")]
@@ -718,7 +767,7 @@ class ShallowWaterSolver:
 
     def _dt_slot(self):
         """Device slot holding the dt of the current state (computed if stale)."""
-        slot = self._dt_buf[self._cur:self._cur + 1]
+        slot = self._slot()
         if self._dt_key != self._state_key():
             q = self._q()
             if "cell_vtx" in self._dm.t:
@@ -758,7 +807,7 @@ class ShallowWaterSolver:
         gr = _lib.p4([_p(self.h.dev("gradcellx")), _p(self.h.dev("gradcelly")), _p(self.hc.dev("gradcellx")),
                       _p(self.hc.dev("gradcelly"))])
         _lib.call("mb_explicitscheme_convective_sw", self._dm.struct, rez, q, g, gr, _p(self.hc.dev("psi")),
-                  float(self.grav), int(self.order), _p(self._ff), self._stream())
+                  float(self.grav), int(self.order), _p(self._face_flux()), self._stream())
 
     def update_term_source(self):
         """manapy/solvers/shallowater/system.py:217-227."""
@@ -819,14 +868,20 @@ class ShallowWaterSolver:
         if self._spare is None:
             self._spare = [torch.empty_like(t) for t in qin]
         qout = self._spare
-        cur = self._use_dt()
-        nxt = self._dt_buf[1 - self._cur:2 - self._cur]
-        _lib.call("mb_sw_step_ex", self._dm.struct, _lib.p5([_p(t) for t in qin] + [_p(z)]),
-                  _lib.p5([_p(t) for t in qout] + [_p(z)]), float(self.cfl), float(self.grav), int(self.order),
-                  _lib.WALLS[self.walls], _p(self._scratch) if self._scratch is not None else None, _p(self._ff),
-                  _p(cur), _p(nxt), self._stream())
+        cur, nxt = self._use_dt(), self._slot(1)
+        q = _lib.p5([_p(t) for t in qin] + [_p(z)])
+        scratch = _p(self._scratch) if self._scratch is not None else None
+        if self._tiles is not None:
+            _lib.call("mb_sw_step_tile", self._dm.struct, self._tiles, q, _lib.p4([_p(t) for t in qout]),
+                      float(self.cfl), float(self.grav), int(self.order), _lib.WALLS[self.walls], scratch, _p(cur),
+                      _p(nxt), _p(self._slot(2)), self._stream())
+            self._ff_step = (float(self.cfl), float(self.grav))
+        else:
+            _lib.call("mb_sw_step_ex", self._dm.struct, q, _lib.p5([_p(t) for t in qout] + [_p(z)]), float(self.cfl),
+                      float(self.grav), int(self.order), _lib.WALLS[self.walls], scratch, _p(self._face_flux()),
+                      _p(cur), _p(nxt), self._stream())
         self._spare = [self.varbs[k].swap_cell(t) for k, t in zip(names, qout)]
-        self._cur = 1 - self._cur
+        self._cur = (self._cur + 1) % 4
         self._dt_key = self._state_key()
         self._dt_host = None
 
@@ -859,14 +914,22 @@ class ShallowWaterSolver:
         qin, z = self._f32_state()
         qout = self._q32[1 - self._q32_i]
         cur = self._use_dt()
-        nxt = self._dt_buf[1 - self._cur:2 - self._cur]
+        nxt = self._slot(1)
         k0 = self._q32_i
         _lib.call("mb_sw_step_f32c_ex", self._dm.struct, _lib.p5([_p(t) for t in qin] + [_p(z)]),
                   _lib.p5([_p(t) for t in qout] + [_p(z)]), _lib.p4([_p(t) for t in self._lo32[k0]]),
                   _lib.p4([_p(t) for t in self._lo32[1 - k0]]), float(self.cfl), float(self.grav), int(self.order),
                   _lib.WALLS[self.walls], _p(self._ff32), _p(cur), _p(nxt), self._stream())
         self._q32_i = 1 - k0
-        for k, buf, lo in zip(self._NAMES[:4], qout, self._lo32[1 - k0]):
+        self._f32_publish()
+        self._cur = (self._cur + 1) % 4
+        self._dt_key = self._state_key()
+        self._dt_host = None
+
+    def _f32_publish(self):
+        """Make the current FP32 state the variables' cell arrays (converted on first read)."""
+        i = self._q32_i
+        for k, buf, lo in zip(self._NAMES[:4], self._q32[i], self._lo32[i]):
             var = self.varbs[k]
 
             def materialise(var=var, buf=buf, lo=lo):
@@ -876,9 +939,6 @@ class ShallowWaterSolver:
             var._s.version["cell"] += 1
             var.set_lazy("cell", materialise)
         self._q32_key = self._keys()
-        self._cur = 1 - self._cur
-        self._dt_key = self._state_key()
-        self._dt_host = None
 
     def check(self):
         """Raise if h, hu, hv or hc holds NaN or infinity, or h is negative (a dry-out the
@@ -911,15 +971,25 @@ class ShallowWaterSolver:
         if self.precision == "fp32c" and self._q32 is not None:
             ff = self._ff32.view(-1, 4)[:, 0]
         else:
-            ff = self._ff.view(-1)[:4 * dm.nbfaces].view(-1, 4)[:, 0]
+            if self._ff_step is not None:
+                # the one-launch step keeps no face fluxes: those of its input state (the same bits)
+                z = self.Z.dev("cell")
+                now = [self.varbs[k].dev("cell") for k in ("h", "hu", "hv", "hc")]
+                _lib.call("mb_sw_step_split", dm.struct, _lib.p5([_p(t) for t in self._spare] + [_p(z)]),
+                          _lib.p5([_p(t) for t in now] + [_p(z)]), *self._ff_step, int(self.order),
+                          _lib.WALLS[self.walls], _p(self._scratch) if self._scratch is not None else None,
+                          _p(self._face_flux()), _p(self._slot()), None, 0, 0, self._stream())
+                self._ff_step = None
+            ff = self._face_flux().view(-1)[:4 * dm.nbfaces].view(-1, 4)[:, 0]
         return float(ff.index_select(0, self._bfaces).double().sum().item())
 
     def launches_per_step(self):
-        """Kernel launches of one fused step: face fluxes, cells (+ next dt), [gradients]."""
-        return 2 + int(self.order == 2)
+        """Kernel launches of one fused step: the step on tiles, or face fluxes and cells (+ next
+        dt); [gradients]."""
+        return (2 if self._tiles is None else 1) + int(self.order == 2)
 
     def release_graphs(self):
-        return None
+        self._graphs.clear()
 
     def advance(self, nsteps):
         """``nsteps`` fused steps on the device, without host synchronisation (each step's dt
@@ -927,8 +997,53 @@ class ShallowWaterSolver:
         self._setup()
         if not self._all_neumann():
             raise NotImplementedError("advance() runs the fused step, which needs Neumann boundaries")
-        for _ in range(int(nsteps)):
+        n = int(nsteps)
+        # a length asked for before is replayed from a graph: after 4 k steps every buffer and the dt
+        # ring are where they were
+        steps = n & ~3
+        if steps:
+            key = (steps,) + self._prime()
+            g = self._graphs.get(key)
+            if g is not None:
+                g.replay()
+                self._published()
+                n -= steps
+            elif self._graphs.worth(key):
+                def body():
+                    for _ in range(steps):
+                        self._fused_step()
+                self._graphs.capture(key, self._dm.device, body).replay()
+                n -= steps
+        for _ in range(n):
             self._fused_step()
+
+    def _prime(self):
+        """All that a step does besides its launches (uploads of host edits, buffers, the dt of the
+        state), done now; returns what the launches of a step depend on."""
+        if self.precision == "fp32c":
+            q, z = self._f32_state()
+            ptrs = [q, self._q32[1 - self._q32_i], [z]]
+        else:
+            q = [self.varbs[k].dev("cell") for k in ("h", "hu", "hv", "hc")]
+            if self._spare is None:
+                self._spare = [torch.empty_like(t) for t in q]
+            if self._tiles is None:
+                self._face_flux()
+            ptrs = [q, self._spare, [self.Z.dev("cell")]]
+        self._use_dt()
+        return (self._cur, float(self.cfl), float(self.grav)) + tuple(_p(t) for ts in ptrs for t in ts)
+
+    def _published(self):
+        """After replayed steps: the state in the buffers it was in is a new one."""
+        if self.precision == "fp32c":
+            self._f32_publish()
+        else:
+            for k in ("h", "hu", "hv", "hc"):
+                self.varbs[k]._s.version["cell"] += 1
+            if self._tiles is not None:
+                self._ff_step = (float(self.cfl), float(self.grav))
+        self._dt_key = self._state_key()
+        self._dt_host = None
 
 
 class EulerSolver:
@@ -983,10 +1098,8 @@ class EulerSolver:
     # ------------------------------------------------------------ state
     def _setup(self):
         if self._dm is None:
-            from . import boundary as B
             for k, v in self.varbs.items():
-                kind = v.resolved_bc.kind
-                if np.any((kind != B.G_NEUMANN) & (kind != B.G_NONE)):
+                if not v.resolved_bc.all_neumann:
                     raise NotImplementedError("Euler boundaries other than manapy's Neumann rule (%s)" % k)
             if np.any(np.asarray(self.domain.host_arrays["faces_name"]) == 10):
                 raise NotImplementedError("halo faces: the Euler step runs on a single-rank mesh")
