@@ -346,6 +346,68 @@ int mb_advdiff_step_tile(const mb_mesh *m, const mb_tiles *t, const mb_bc *bc, c
                          const double *w_in, double *w_out, const double *sign_cf, const double *coef,
                          const double *src, const double *dt_dev, void *stream);
 
+/* Tiles of a tetrahedral mesh for the second-order step: local cells of a tile are its own, then at
+ * cells + e the outside cells ext[e] that share a vertex with them; local nodes and edges are
+ * those of its cells.  Coordinates are relative to the centre of the tile's first cell. */
+#define MB_TET_TILE_MAX_CELLS 512
+typedef struct mb_tet_tiles {
+  int32_t cells, count;          /* cells per tile (even, 32 .. MB_TET_TILE_MAX_CELLS), ceil(nbcells / cells) tiles */
+  int32_t ext_cap, node_cap, edge_cap;   /* strides: >= outside cells (even), >= local nodes, >= local edges */
+  int32_t ngrp_cap, egrp_cap;    /* >= groups of 32 nodes / edges + 1, multiples of 4 */
+  int32_t ninc_cap, einc_cap;    /* >= entries of the node / edge lists, multiples of 32 */
+  int32_t pad_;
+  /* every table starts on 32 bytes */
+  int32_t *head;                 /* [count][8] outside cells, nodes, edges, node and edge list entries, 0, 0, 0 */
+  int32_t *ext;                  /* [count][ext_cap] outside cells */
+  double *ext_xy, *ext_z;        /* [count][ext_cap][2], [count][ext_cap] their relative centres */
+  double *own_xy, *own_z;        /* [nbcells][2], [nbcells] relative centres of the tiles' own cells */
+  int32_t *node;                 /* [count][node_cap] vertex; bit 30: this tile writes its value, 29: boundary faces */
+  double *node_mu;               /* [nbnodes][4] centre -> vertex weights of the sums: mu_x, mu_y, mu_z, a */
+  double *node_kappa;            /* [nbnodes] sum of its weights over its cells */
+  int32_t *ngrp, *egrp;          /* [count][ngrp_cap], [count][egrp_cap] offsets of the lists of 32 nodes / edges */
+  uint16_t *ninc, *einc;         /* node / edge -> local cells, SELL-32; cells + ext_cap past a list's end */
+  uint16_t *cell;                /* [nbcells][16] local nodes (4), local edges (6), local neighbours (4; 0xffff:
+                                    boundary face), 1 if the cell has stencil ghosts, 0 */
+  double *cell_q;                /* [12][nbcells] least-squares reconstruction at three faces */
+  uint16_t *link;                /* [nbcells] bit j left cell of face j, bits 4+2j.. the face in the neighbour */
+} mb_tet_tiles;
+
+/* Set-up, once per mesh (compact tables, cell_lsq and the edge tables needed): head [count][8], *status as
+ * mb_tile_sizes; then every table of t. */
+int mb_tet_tile_sizes(const mb_mesh *m, int32_t cells, int32_t *head, int32_t *status, void *stream);
+int mb_tet_tile_fill(const mb_mesh *m, const mb_tet_tiles *t, void *stream);
+/* Bytes of shared memory a block of the gradient pass takes with the strides of t. */
+int mb_tet_tile_bytes(const mb_tet_tiles *t);
+/* The diffusive flux sum of every tetrahedron as a linear form, [8][nbcells]: c_1, c_2, c_3 of the vertex
+ * differences V_k - V_0, B_0..B_3 of the value differences across the faces, 1 / volume. */
+int mb_tet_coef(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_params *p, double *coef, void *stream);
+/* mb_advdiff_step (manapy/solvers/advecdiff/system.py:156-172) at second order on the tiles of a
+ * tetrahedral mesh, in two launches: gradients, limiter and face values (and vertex values) per
+ * tile; fluxes and update per cell.  Equal to it up to rounding.  face_values: 4 nbcells doubles,
+ * 32-byte aligned; node_scratch: nbnodes (diffusion); sign_cf 32-byte aligned; coef from mb_tet_coef
+ * ([8][nbcells]; diffusion). */
+int mb_advdiff_step_tet(const mb_mesh *m, const mb_tet_tiles *t, const mb_bc *bc, const mb_advdiff_params *p,
+                        const double *w_in, double *w_out, const double *sign_cf, const double *coef,
+                        const double *src, const double *dt_dev, double *face_values, double *node_scratch,
+                        void *stream);
+
+/* The same step for large tetrahedral meshes, in three launches: vertex and edge sums in memory, face
+ * values per cell, fluxes.  mb_tet_tables_fill fills cell_q and link (as in mb_tet_tiles), node_mu
+ * ([nbnodes][4] mu_x, mu_y, mu_z, 1 / den: vertex weights of the sums relative to the vertex, 32-byte
+ * aligned); *status (device, zero before) becomes 1 where two cells share two faces (unsupported).
+ * rows as mb_advdiff_step_rows; scratch: 4 (nbcells + nbnodes + nbedges) doubles, 32-byte aligned. */
+typedef struct mb_tet_tables {
+  double *cell_q;
+  uint16_t *link;
+  double *node_mu;
+  int32_t *status;
+} mb_tet_tables;
+int mb_tet_tables_fill(const mb_mesh *m, const mb_tet_tables *t, void *stream);
+int mb_advdiff_step_tet_sums(const mb_mesh *m, const mb_tet_tables *t, const mb_bc *bc, const mb_advdiff_params *p,
+                             const double *w_in, double *w_out, const double *rows_in, double *rows_out,
+                             const double *sign_cf, const double *coef, const double *src, const double *dt_dev,
+                             double *scratch, double *node_scratch, void *stream);
+
 /* Rows {centre, value} of a state, [nbcells][4] doubles, 32-byte aligned: {x, y, w, 0} for
  * triangles, {x, y, z, w} for tetrahedra (no counterpart in manapy). */
 int mb_pack_rows(const mb_mesh *m, const double *w, double *rows, void *stream);

@@ -62,6 +62,18 @@ class MbFaceTiles(ctypes.Structure):
                 ("face", _vp), ("face_n0", _vp), ("face_n1", _vp), ("face_mes", _vp), ("cell", _vp), ("cell_ns", _vp)]
 
 
+class MbTetTiles(ctypes.Structure):
+    _fields_ = [("cells", _i32), ("count", _i32), ("ext_cap", _i32), ("node_cap", _i32), ("edge_cap", _i32),
+                ("ngrp_cap", _i32), ("egrp_cap", _i32), ("ninc_cap", _i32), ("einc_cap", _i32), ("pad_", _i32),
+                ("head", _vp), ("ext", _vp), ("ext_xy", _vp), ("ext_z", _vp), ("own_xy", _vp), ("own_z", _vp),
+                ("node", _vp), ("node_mu", _vp), ("node_kappa", _vp), ("ngrp", _vp), ("egrp", _vp), ("ninc", _vp),
+                ("einc", _vp), ("cell", _vp), ("cell_q", _vp), ("link", _vp)]
+
+
+class MbTetTables(ctypes.Structure):
+    _fields_ = [("cell_q", _vp), ("link", _vp), ("node_mu", _vp), ("status", _vp)]
+
+
 class MbAdvDiffItem(ctypes.Structure):
     _fields_ = [("m", MbMesh), ("bc", MbBC), ("p", MbAdvDiffParams), ("w", _vp * 2), ("lo", _vp * 2), ("sign_cf", _vp),
                 ("src", _vp), ("dt_dev", _vp), ("cell_scratch", _vp), ("node_scratch", _vp),
@@ -161,6 +173,15 @@ _SIGS = {
     "mb_face_tile_sizes": [_M, _i32, _vp, _vp, _vp],
     "mb_face_tile_fill": [_M, ctypes.POINTER(MbFaceTiles), _vp],
     "mb_sw_step_tile": [_M, ctypes.POINTER(MbFaceTiles), _P5, _P4, _d, _d, _i32, _i32, _vp, _vp, _vp, _vp, _vp],
+    "mb_tet_tile_sizes": [_M, _i32, _vp, _vp, _vp],
+    "mb_tet_tile_fill": [_M, ctypes.POINTER(MbTetTiles), _vp],
+    "mb_tet_tile_bytes": [ctypes.POINTER(MbTetTiles)],
+    "mb_tet_coef": [_M, _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp],
+    "mb_advdiff_step_tet": [_M, ctypes.POINTER(MbTetTiles), _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp, _vp,
+                            _vp, _vp, _vp, _vp, _vp],
+    "mb_tet_tables_fill": [_M, ctypes.POINTER(MbTetTables), _vp],
+    "mb_advdiff_step_tet_sums": [_M, ctypes.POINTER(MbTetTables), _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp,
+                                 _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "mb_tile_bytes": [ctypes.POINTER(MbTiles)],
     "mb_tile_coef": [_M, _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp],
     "mb_advdiff_step_tile": [_M, ctypes.POINTER(MbTiles), _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp, _vp,

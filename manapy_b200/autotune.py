@@ -90,7 +90,7 @@ def launch_variant(solver, steps=64):
     s._setup()
     dm = s._dm
     if not (s.precision == "fp64" and s.order == 2 and s.diffusion and "cell_vtx" in dm.t) or \
-            dm.nbcells < SMALL or s._tiles is not None:
+            dm.nbcells < SMALL or s._tiles is not None or s._tables is not None:
         return 0
     k = ("variant",) + _key(s)
     if k in _cache:

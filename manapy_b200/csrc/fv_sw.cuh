@@ -6,7 +6,7 @@
 // takes the two-launch step in parts, equals the single-domain run that takes the tiles.
 #pragma once
 
-#include "fv_compact.cuh"
+#include "fv_tile.cuh"
 
 namespace mb {
 
@@ -91,9 +91,9 @@ __device__ __forceinline__ void srnh0(double hu_l, double hu_r, double hv_l, dou
 __device__ __forceinline__ void sw_reconstruct(const double *const gr[4], const double *psi, const double *cc, int c,
                                                double fx, double fy, double &h, double &hc) {
   const double r0 = sws(fx, ld(cc + 3 * (long long)c)), r1 = sws(fy, ld(cc + 3 * (long long)c + 1));
-  const double p = ld(psi + c);
-  h = swf(p, swd(ld(gr[0] + c), r0, ld(gr[1] + c), r1), h);
-  hc = swf(p, swd(ld(gr[2] + c), r0, ld(gr[3] + c), r1), hc);
+  const double p = ld_after(psi + c);
+  h = swf(p, swd(ld_after(gr[0] + c), r0, ld_after(gr[1] + c), r1), h);
+  hc = swf(p, swd(ld_after(gr[2] + c), r0, ld_after(gr[3] + c), r1), hc);
 }
 
 // Momentum of a reflective-wall ghost: the interior momentum with its normal component

@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(kSwTileThreads, MB_SW_TILE_MIN_BLOCKS)
 #pragma unroll
     for (int k = 0; k < 5; ++k) {
       tile_bulk(q + k * Q, a.q[k] + c0, 8u * (nc & ~1), bar);
-      if (nc & 1) q[k * Q + nc - 1] = a.q[k][c0 + nc - 1];
+      if (nc & 1) q[k * Q + nc - 1] = ld_after(a.q[k] + c0 + nc - 1);
     }
     if (b == 0) *a.dt_after = 1e6;
   }
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kSwTileThreads, MB_SW_TILE_MIN_BLOCKS)
   }
   __syncthreads();
 
-  const double dt = *a.dt_cur;
+  const double dt = ld_after(a.dt_cur);
   double best = 1e300;
   for (int k = tid; k < nc; k += kSwTileThreads) {
     const int i = c0 + k;
@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(kSwTileThreads, MB_SW_TILE_MIN_BLOCKS)
       // where the cell has a boundary face, cells.cellfid slot j is not the cell across face j
       if ((c.fl & kTileRim) && s.inner[j]) {
         const int g = ld(m.cell_cellfid + 4 * (long long)i + j);
-        s.hp[j] = a.q[0][g];
-        s.zp[j] = a.q[4][g];
+        s.hp[j] = ld_after(a.q[0] + g);
+        s.zp[j] = ld_after(a.q[4] + g);
       }
     }
     double h, hu, hv, hc;

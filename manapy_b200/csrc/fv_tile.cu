@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(kTileThreads, MB_TILE_MIN_BLOCKS)
   const int nc = min(T, m.nbcells - c0);
   const int4 head = __ldg(reinterpret_cast<const int4 *>(t.head) + b);
   const int n1 = head.x, next = head.y, nn = head.z;
-  const GhostRule ghost = make_rule(m, bc, w);
+  const GhostAfter ghost{make_rule(m, bc, w)};
   const int32_t *ext = t.ext + (long long)b * t.ext_cap;
   const int32_t *node = t.node + (long long)b * t.node_cap;
 
@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(kTileThreads, MB_TILE_MIN_BLOCKS)
   tile_after_previous();
   if (tid == 0) {
     tile_bulk(cw, w + c0, 8u * (nc & ~1), bar);
-    if (nc & 1) cw[nc - 1] = w[c0 + nc - 1];
+    if (nc & 1) cw[nc - 1] = ld_after(w + c0 + nc - 1);
   }
   for (int k = tid; k < next; k += kTileThreads) tile_copy8(cw + T + k, w + (k == tid ? first : ld(ext + k)));
   tile_copies_done();
@@ -162,8 +162,15 @@ __global__ void __launch_bounds__(kTileThreads, MB_TILE_MIN_BLOCKS)
       if (cnt & kNodeGhosts) {
         const int v = ld(node + k);
         a += (ld(t.node_kappa + v) - 1.) * W;
-        for (int q = ld(m.n2g_ptr + v); q < ld(m.n2g_ptr + v + 1); ++q)
-          a += ld(m.n2g_alpha + q) * ghost(ld(m.n2g_idx + q));
+        const int e = ld(m.n2g_ptr + v + 1);
+        for (int q = ld(m.n2g_ptr + v); q < e; q += 4) {
+          int f[4];
+          double g[4];
+          ghost4(ghost.g, m.n2g_idx, q, e, f, g);
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if (f[u] >= 0) a += ld(m.n2g_alpha + q + u) * g[u];
+        }
       }
       nv[k] = a;
     }
@@ -203,11 +210,18 @@ __global__ void __launch_bounds__(kTileThreads, MB_TILE_MIN_BLOCKS)
       }
       if (c.fl & kTileGhosts) {
         const int i = k < nc ? c0 + k : ld(ext + k - nc);
-        for (int q = ld(m.ghostnid_ptr + i); q < ld(m.ghostnid_ptr + i + 1); ++q) {
-          const int f = ld(m.ghostnid_idx + q);
-          const double d = ghost(f) - wi;
-          jx += (ld(m.face_ghostcenter + 3 * (long long)f) - ci.x) * d;
-          jy += (ld(m.face_ghostcenter + 3 * (long long)f + 1) - ci.y) * d;
+        const int e = ld(m.ghostnid_ptr + i + 1);
+        for (int q = ld(m.ghostnid_ptr + i); q < e; q += 4) {
+          int f[4];
+          double g[4];
+          ghost4(ghost.g, m.ghostnid_idx, q, e, f, g);
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            if (f[u] < 0) continue;
+            const double d = g[u] - wi;
+            jx += (ld(m.face_ghostcenter + 3 * (long long)f[u]) - ci.x) * d;
+            jy += (ld(m.face_ghostcenter + 3 * (long long)f[u] + 1) - ci.y) * d;
+          }
         }
       }
       // reconstruction offsets g . (face centre - centre) at the three faces; they sum to zero
@@ -232,7 +246,7 @@ __global__ void __launch_bounds__(kTileThreads, MB_TILE_MIN_BLOCKS)
     __syncthreads();
   }
 
-  const double dt = *dt_dev;
+  const double dt = ld_after(dt_dev);
 #pragma unroll 2
   for (int k = tid; k < nc; k += kTileThreads) {
     const int i = c0 + k;
@@ -279,7 +293,7 @@ __global__ void __launch_bounds__(kTileThreads, MB_TILE_MIN_BLOCKS)
       acc += own ? -F : F;
       if (DF) acc += B[j] * (wo - wi);
     }
-    w_out[i] = wi + dt * (acc * rv + (src ? ld(src + i) : 0.0));
+    w_out[i] = wi + dt * (acc * rv + (src ? ld_after(src + i) : 0.0));
   }
 }
 

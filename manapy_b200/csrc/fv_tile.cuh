@@ -93,10 +93,78 @@ inline bool face_tiles_ok(const mb_mesh *m, const mb_face_tiles *t) {
   return true;
 }
 
+inline bool tet_tiles_ok(const mb_mesh *m, const mb_tet_tiles *t) {
+  if (!t || t->cells < 32 || (t->cells & 1) || t->cells > MB_TET_TILE_MAX_CELLS ||
+      t->count != ceil_div(m->nbcells, t->cells) || t->ext_cap < 0 || (t->ext_cap & 1) || t->node_cap < 1 ||
+      t->edge_cap < 1 || (t->ngrp_cap & 3) || (t->egrp_cap & 3) || t->ngrp_cap < ceil_div(t->node_cap, 32) + 1 ||
+      t->egrp_cap < ceil_div(t->edge_cap, 32) + 1 || t->ninc_cap < 32 || (t->ninc_cap & 31) || t->einc_cap < 32 ||
+      (t->einc_cap & 31))
+    return false;
+  const void *p[] = {t->head, t->ext, t->ext_xy, t->ext_z, t->own_xy, t->own_z, t->node, t->node_mu, t->node_kappa,
+                     t->ngrp, t->ninc, t->egrp, t->einc, t->cell, t->cell_q, t->link};
+  for (const void *q : p)
+    if (!q || ((uintptr_t)q & 31)) return false;
+  return true;
+}
+// a tetrahedral tile's node entry: the vertex, and
+constexpr int kTetOwned = 1 << 30;    // this tile writes its value
+constexpr int kTetGhosts = 1 << 29;   // it has boundary faces
+
 // programmatic dependent launch: a step's blocks may start while the previous step's last ones
 // run; before tile_after_previous() they touch only tables that no step writes
 __device__ __forceinline__ void tile_let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void tile_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Loads of what an earlier launch wrote.  The read-only path (ld, const __restrict__) may be moved
+// above tile_after_previous() by the compiler, since it promises that nothing writes the data
+// while the kernel runs; these are not.
+__device__ __forceinline__ double ld_after(const double *p) {
+  double v;
+  asm volatile("ld.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void ld4_after(const double *p, double &a, double &b, double &c, double &d) {
+  asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p) : "memory");
+}
+// GhostRule with the state loaded so
+struct GhostAfter {
+  GhostRule g;
+  __device__ __forceinline__ double operator()(int f) const {
+    const int k = g.kind[f];
+    if (k == MB_G_DIRICHLET) return ld(g.value + f);
+    const double wc = ld_after(g.w + ld(g.face_cellid + 2 * (long long)f));
+    if (k == MB_G_NEUMANN) return wc;
+    if (k == MB_G_NONSLIP) return -1 * wc;
+    if (k == MB_G_NEUMANN_NH) return wc + ld(g.value + f) * ld(g.dist + f);
+    if (k == MB_G_CELL_AT_FACE) return ld_after(g.w + (long long)ld(g.value + f));
+    return 0.0;
+  }
+};
+
+// Ghost values of the boundary faces idx[q .. min(q + 4, e)): the four chains index -> rule, cell -> value
+// run side by side (one after the other, the lists of boundary vertices and cells were the longest
+// chain of a small mesh's step).  f < 0 and v = 0 past the end.
+__device__ __forceinline__ void ghost4(const GhostRule &g, const int32_t *idx, int q, int e, int f[4], double v[4]) {
+  int k[4], c[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) f[u] = q + u < e ? ld(idx + q + u) : -1;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const long long at = f[u] < 0 ? 0 : f[u];
+    k[u] = f[u] < 0 ? MB_G_NONE : (int)g.kind[at];
+    v[u] = ld(g.value + at);
+    c[u] = ld(g.face_cellid + 2 * at);
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int k_ = k[u];
+    const double val = v[u];
+    double wc = 0.;
+    if (k_ != MB_G_NONE && k_ != MB_G_DIRICHLET) wc = ld_after(g.w + (k_ == MB_G_CELL_AT_FACE ? (long long)val : c[u]));
+    v[u] = k_ == MB_G_DIRICHLET ? val : (k_ == MB_G_NONSLIP ? -1 * wc : wc);
+    if (k_ == MB_G_NEUMANN_NH) v[u] = wc + val * ld(g.dist + f[u]);
+  }
+}
 
 template <class... P, class... A>
 inline cudaError_t tile_launch(void (*k)(P...), int blocks, int threads, int bytes, cudaStream_t st, A... args) {

@@ -1,53 +1,11 @@
 // Builds the tiles of a triangle mesh (fv_tile.cuh) on the device: one block per tile, two
 // passes (sizes, then the tables at strides the caller chose from the sizes).  Set-up work,
 // once per mesh.
-#include "fv_tile.cuh"
+#include "fv_tile_plan.cuh"
 
 namespace mb {
 
 constexpr int kHashCells = 4096, kHashNodes = 2048, kMaxOut = 2048, kMaxNodes = 1536;
-
-__device__ __forceinline__ unsigned tile_hash(int key, int mask) { return ((unsigned)key * 2654435761u >> 15) & mask; }
-
-// key's slot, inserting it if absent (was_new); -1 when the table is full
-__device__ int hash_put(int *keys, int cap, int key, bool &was_new) {
-  unsigned h = tile_hash(key, cap - 1);
-  was_new = false;
-  for (int probe = 0; probe < cap; ++probe, h = (h + 1) & (cap - 1)) {
-    const int old = atomicCAS(keys + h, -1, key);
-    if (old == -1) { was_new = true; return (int)h; }
-    if (old == key) return (int)h;
-  }
-  return -1;
-}
-__device__ int hash_get(const int *keys, const uint16_t *vals, int cap, int key) {
-  unsigned h = tile_hash(key, cap - 1);
-  for (int probe = 0; probe < cap; ++probe, h = (h + 1) & (cap - 1)) {
-    if (keys[h] == key) return vals[h];
-    if (keys[h] == -1) break;
-  }
-  return 0;
-}
-
-// ascending sort of a[0, n) by the block (bitonic, padded to a power of two with INT_MAX; the
-// array has room for it)
-__device__ void block_sort(int *a, int n) {
-  int p = 1;
-  while (p < n) p <<= 1;
-  for (int i = n + threadIdx.x; i < p; i += blockDim.x) a[i] = 0x7fffffff;
-  __syncthreads();
-  for (int k = 2; k <= p; k <<= 1)
-    for (int j = k >> 1; j > 0; j >>= 1) {
-      for (int i = threadIdx.x; i < p; i += blockDim.x) {
-        const int q = i ^ j;
-        if (q > i) {
-          const int x = a[i], y = a[q];
-          if ((x > y) == ((i & k) == 0)) { a[i] = y; a[q] = x; }
-        }
-      }
-      __syncthreads();
-    }
-}
 
 struct TileShared {
   int ckey[kHashCells];
@@ -224,7 +182,10 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_plan(mb_mesh m, mb_tiles 
   }
 }
 
+// A step launched next may read its tables before it waits for its predecessor in the stream: that
+// predecessor is this launch, which waits for the tables.
 __global__ void k_tile_filled() {}
+void tile_filled(cudaStream_t st) { k_tile_filled<<<1, 32, 0, st>>>(); }
 
 // inverse of the least-squares moment matrix of every cell (manapy/ast/functions2d.py:5-104),
 // summed over the lsq_sell slots and the stencil ghosts: {i_yy, -i_xy, i_xx} / det, 0
@@ -495,9 +456,7 @@ int mb_tile_fill(const mb_mesh *m, const mb_tiles *t, double *scratch, void *str
   k_tile_node<<<ceil_div(m->nbnodes, kBlock), kBlock, 0, st>>>(*m, node_w, t->node_kappa);
   const int rc = run_plan<true>(m, t, nullptr, nullptr, minv, node_w, st);
   if (rc != MB_OK) return rc;
-  // a step launched next may read the tables before it waits for its predecessor in the stream:
-  // that predecessor is this launch, which waits for the tables
-  k_tile_filled<<<1, 32, 0, st>>>();
+  tile_filled(st);
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
 }
 
@@ -537,7 +496,7 @@ int mb_face_tile_fill(const mb_mesh *m, const mb_face_tiles *t, void *stream) {
   if (face_mesh_bad(m) || !face_tiles_ok(m, t)) return MB_EINVAL;
   const int rc = run_face_plan<true>(m, t, nullptr, nullptr, ST(stream));
   if (rc != MB_OK) return rc;
-  k_tile_filled<<<1, 32, 0, ST(stream)>>>();
+  tile_filled(ST(stream));
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
 }
 

@@ -504,7 +504,87 @@ class DeviceMesh:
                                          "cell_ns": 16 * self.nbcells}, head),
                    _lib.call("mb_face_tile_fill", self.struct, t, st))
 
-    def _carve(self, t, sizes, head):
+    # Tetrahedra, second order (fv_tet_tile.cu): a B200 runs 148 SMs x 2 blocks of the tiled gradient pass
+    # at once; tiles of one or two rounds of blocks, at most 256 cells (shared memory).  A tile has
+    # three to five outside cells per cell of its own, so past two rounds the sums in memory are as
+    # fast (16,464 cells: 15.4 against 25.5 us; 93,750: 32.7 / 38.0; 162,000: 50.2 / 50.5; 384,000:
+    # 100 / 83)
+    TET_SLOTS = 296
+    TET_TILE_CELLS = 256
+    TET_TILED = 110_000
+
+    @classmethod
+    def tet_tile_cells(cls, nbcells):
+        rounds = -(-int(nbcells) // (cls.TET_SLOTS * cls.TET_TILE_CELLS))
+        return min(cls.TET_TILE_CELLS, max(96, 16 * -(-int(nbcells) // (16 * cls.TET_SLOTS * rounds))))
+
+    def tet_tiles(self, stream=None, cells=None):
+        """The tiles of a tetrahedral mesh (``_lib.MbTetTiles``), built on the device on first use (with
+        ``cell_lsq`` and the edge tables in the struct); None where the tiled second-order step
+        does not apply."""
+        cells = self.tet_tile_cells(self.nbcells) if cells is None else int(cells)
+        if getattr(self, "_tet_tiles", None) is None:
+            self._tet_tiles = {}
+        if cells not in self._tet_tiles:
+            self._tet_tiles[cells] = self._build_tet_tiles(cells, stream)
+        got = self._tet_tiles[cells]
+        return None if got is None else got[0]
+
+    def _build_tet_tiles(self, cells, stream):
+        need = ("cell_vtx", "cell_xy", "n2c_ptr", "n2c_alpha", "n2g_ptr", "ghostnid_ptr", "face_ghostcenter", "cell_lsq",
+                "cell_edges", "edge_sell_idx")
+        if self.dim != 3 or self.device is None or self.stencil != "shared" or any(n not in self.t for n in need):
+            return None
+        dev = self.device
+        st = stream if stream is not None else torch.cuda.current_stream(dev).cuda_stream
+        count = -(-self.nbcells // cells)
+        head = torch.empty(8 * count + 8, dtype=torch.int32, device=dev)
+        status = head[8 * count:]
+        status.zero_()
+        _lib.call("mb_tet_tile_sizes", self.struct, cells, head.data_ptr(), status.data_ptr(), st)
+        ext, nodes, edges, ninc, einc, _, _, _, bad = torch.cat([torch.amax(head[:8 * count].view(-1, 8), 0),
+                                                                status[:1]]).tolist()
+        if bad:
+            return None
+        up = lambda n, k: -(-n // k) * k  # noqa: E731
+        t = _lib.MbTetTiles()
+        t.cells, t.count, t.ext_cap, t.node_cap, t.edge_cap = cells, count, up(ext, 2), nodes, edges
+        t.ngrp_cap, t.egrp_cap = up(-(-nodes // 32) + 1, 4), up(-(-edges // 32) + 1, 4)
+        t.ninc_cap, t.einc_cap = up(ninc, 32), up(einc, 32)
+        if _lib.lib().mb_tet_tile_bytes(t) > self.TILE_BYTES:
+            return None
+        nc, nn = self.nbcells, self.nbnodes
+        buf = self._carve(t, {"ext": 4 * count * t.ext_cap, "ext_xy": 16 * count * t.ext_cap,
+                              "ext_z": 8 * count * t.ext_cap, "own_xy": 16 * nc, "own_z": 8 * nc,
+                              "node": 4 * count * nodes, "node_mu": 32 * nn, "node_kappa": 8 * nn,
+                              "ngrp": 4 * count * t.ngrp_cap, "egrp": 4 * count * t.egrp_cap,
+                              "ninc": 2 * count * t.ninc_cap, "einc": 2 * count * t.einc_cap, "cell": 32 * nc,
+                              "cell_q": 96 * nc, "link": 2 * nc}, head)
+        _lib.call("mb_tet_tile_fill", self.struct, t, st)
+        return t, (head, buf)
+
+    def tet_tables(self, stream=None):
+        """The tables of the second-order step on large tetrahedral meshes (``_lib.MbTetTables``), built on
+        the device on first use (with ``cell_lsq`` and the edge tables in the struct); None where it
+        does not apply."""
+        if getattr(self, "_tet_tables", None) is None:
+            need = ("cell_lsq", "cell_edges", "edge_sell_idx", "n2c_sum_idx", "n2c_ptr", "n2c_alpha", "n2g_ptr",
+                    "ghostnid_ptr", "face_ghostcenter")
+            self._tet_tables = (None, None)
+            if self.dim == 3 and self.device is not None and self.stencil == "shared" and \
+                    all(n in self.t for n in need):
+                nc, nn = self.nbcells, self.nbnodes
+                status = torch.zeros(1, dtype=torch.int32, device=self.device)
+                t = _lib.MbTetTables()
+                buf = self._carve(t, {"cell_q": 96 * nc, "link": 2 * nc, "node_mu": 32 * nn})
+                t.status = status.data_ptr()
+                st = stream if stream is not None else torch.cuda.current_stream(self.device).cuda_stream
+                _lib.call("mb_tet_tables_fill", self.struct, t, st)
+                if not int(status.item()):
+                    self._tet_tables = (t, (buf, status))
+        return self._tet_tables[0]
+
+    def _carve(self, t, sizes, head=None):
         """One device allocation for the tables of ``t`` (bytes by field), at 256-byte boundaries."""
         up = lambda n: -(-n // 256) * 256  # noqa: E731
         buf = torch.empty(sum(up(n) for n in sizes.values()) + 256, dtype=torch.uint8, device=self.device)
@@ -512,7 +592,8 @@ class DeviceMesh:
         for k, n in sizes.items():
             setattr(t, k, at)
             at += up(n)
-        t.head = head.data_ptr()
+        if head is not None:
+            t.head = head.data_ptr()
         return buf
 
     def upload(self, device, stream=None):

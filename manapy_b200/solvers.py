@@ -202,13 +202,19 @@ class AdvectionDiffusionSolver:
             self._sign = torch.zeros(4 * self._dm.nbcells, dtype=torch.float64, device=dev)
             self._params = _lib.MbAdvDiffParams(int(self.order), int(self.diffusion), float(self.Dxx),
                                                 float(self.Dyy), float(self.Dzz))
-            self._tiles = self._coef = None
+            self._tiles = self._tables = self._coef = None
             if self.precision == "fp64" and self.launch == "auto" and (self.order == 2 or self.diffusion):
-                self._tiles = self._dm.tiles(self._stream())   # triangles: the one-launch step
-            if self._tiles is not None and self.diffusion:
-                self._coef = torch.empty(6 * self._dm.nbcells, dtype=torch.float64, device=dev)
-                _lib.call("mb_tile_coef", self._dm.struct, self.var.device_bc.struct, self._params, _p(self._coef),
-                          self._stream())
+                if self.dim == 2:      # the one-launch step
+                    self._tiles = self._dm.tiles(self._stream())
+                elif self.order == 2 and self.lsq_sums:
+                    if self._dm.nbcells <= self._dm.TET_TILED:
+                        self._tiles = self._dm.tet_tiles(self._stream())
+                    if self._tiles is None:
+                        self._tables = self._dm.tet_tables(self._stream())
+            if (self._tiles or self._tables) is not None and self.diffusion:
+                self._coef = torch.empty((6 if self.dim == 2 else 8) * self._dm.nbcells, dtype=torch.float64, device=dev)
+                _lib.call("mb_tile_coef" if self.dim == 2 else "mb_tet_coef", self._dm.struct,
+                          self.var.device_bc.struct, self._params, _p(self._coef), self._stream())
         return self._dm
 
     def _stream(self):
@@ -336,11 +342,12 @@ class AdvectionDiffusionSolver:
 
     def _scratch(self):
         dm = self._dm
-        if getattr(self, "_cs", None) is None or self._cs.numel() < dm.cell_scratch_size():
-            # 4 nbcells (2D: records) or 8 nbcells (3D: records, rows), plus the vertex and edge
+        need = dm.cell_scratch_size() if self._tiles is None else 4 * dm.nbcells
+        if getattr(self, "_cs", None) is None or self._cs.numel() < need:
+            # 4 nbcells (2D: records; 3D on tiles: face values) or 8 nbcells (3D: records, rows), plus the vertex and edge
             # records when the 3D step uses the edge sums (grown if another solver on this mesh
             # opted the struct into them since)
-            self._cs = torch.empty(dm.cell_scratch_size(), dtype=torch.float64, device=dm.device)
+            self._cs = torch.empty(need, dtype=torch.float64, device=dm.device)
             self._ns = torch.empty(dm.nbnodes, dtype=torch.float64, device=dm.device)
         return self._cs, self._ns
 
@@ -349,7 +356,7 @@ class AdvectionDiffusionSolver:
     def _use_rows(self):
         # tetrahedra only: a triangle's 16-byte centre row shares its 32-byte sector with its
         # Morton neighbour's, so 32-byte rows would double the gathered sectors (measured slower)
-        return self.order == 2 and self.dim == 3 and "cell_vtx" in self._dm.t
+        return self.order == 2 and self.dim == 3 and "cell_vtx" in self._dm.t and self._tiles is None
 
     def _rows_of(self, buf):
         if getattr(self, "_rowbufs", None) is None:
@@ -371,6 +378,17 @@ class AdvectionDiffusionSolver:
     def _call_step(self, w_in, w_out, src, st):
         """The kernels of one FP64 step (the rows of ``w_in`` current where they are used)."""
         dm, bc = self._dm, self.var.device_bc.struct
+        if self._tiles is not None and self.dim == 3:
+            cs, ns = self._scratch()
+            _lib.call("mb_advdiff_step_tet", dm.struct, self._tiles, bc, self._params, _p(w_in), _p(w_out),
+                      _p(self._sign), _p(self._coef), src, _p(self._dt_dev), _p(cs), _p(ns), st)
+            return
+        if self._tables is not None:
+            cs, ns = self._scratch()
+            _lib.call("mb_advdiff_step_tet_sums", dm.struct, self._tables, bc, self._params, _p(w_in), _p(w_out),
+                      _p(self._rows_of(w_in)), _p(self._rows_of(w_out)), _p(self._sign), _p(self._coef), src,
+                      _p(self._dt_dev), _p(cs), _p(ns), st)
+            return
         if self._tiles is not None:
             _lib.call("mb_advdiff_step_tile", dm.struct, self._tiles, bc, self._params, _p(w_in), _p(w_out),
                       _p(self._sign), _p(self._coef), src, _p(self._dt_dev), st)
@@ -487,7 +505,7 @@ class AdvectionDiffusionSolver:
         # two launches: vertex and edge sums, then the cells)
         dm = self._dm
         if dm is not None and self._tiles is not None:
-            return 1
+            return 1 if self.dim == 2 else 2
         sums = dm is not None and self.order == 2 and dm.struct is not None and bool(dm.struct.cell_edges)
         return 1 + int(self.order == 2 or bool(self.diffusion)) + int(sums)
 
@@ -599,7 +617,7 @@ class AdvectionDiffusionSolver:
         if self._graph_bufs is None:
             self._graph_bufs = (var.dev("cell"), self._spare)
         a, b = self._graph_bufs
-        if self._tiles is None:
+        if self._tiles is None or self.dim == 3:
             self._scratch()             # allocated before the capture
         if self._use_rows():
             self._rows_of(a), self._rows_of(b)
