@@ -483,7 +483,7 @@ int mb_cell_face_sign(const mb_mesh *m, const double *u_face, const double *v_fa
 int mb_face_sign(const mb_mesh *m, const double *u_face, const double *v_face,
                  const double *w_face, double *sign_face, void *stream);
 
-/* Tiles of cells with their faces, for the one-launch shallow-water step: local cells as in mb_tiles
+/* Tiles of cells with their faces, for the one-launch shallow-water and Euler steps: local cells as in mb_tiles
  * (the outside cells are those across a face of the tile only), local faces those of the tile's
  * cells. */
 typedef struct mb_face_tiles {
@@ -512,6 +512,10 @@ int mb_face_tile_fill(const mb_mesh *m, const mb_face_tiles *t, void *stream);
 int mb_sw_step_tile(const mb_mesh *m, const mb_face_tiles *t, const double *const q_in[5], double *const q_out[4],
                     double cfl, double grav, int32_t order, int32_t walls, double *scratch, const double *dt_cur,
                     double *dt_next, double *dt_after, void *stream);
+
+/* mb_euler_step_2d in one launch on the tiles of m (bit-identical to it): ring, t and time as there. */
+int mb_euler_step_tile(const mb_mesh *m, const mb_face_tiles *t, const double *const q_in[5], double *const q_out[5],
+                       double cfl, double gamma, double *ring, int step, double *time, void *stream);
 
 /* One shallow-water step (ShallowWaterSolver.compute_fluxes + compute_new_val,
  * manapy/solvers/shallowater/system.py:248-281,237-242) with Neumann ghosts on every

@@ -172,6 +172,7 @@ _SIGS = {
     "mb_tile_fill": [_M, ctypes.POINTER(MbTiles), _vp, _vp],
     "mb_face_tile_sizes": [_M, _i32, _vp, _vp, _vp],
     "mb_face_tile_fill": [_M, ctypes.POINTER(MbFaceTiles), _vp],
+    "mb_euler_step_tile": [_M, ctypes.POINTER(MbFaceTiles), _P5, _P5, _d, _d, _vp, _i32, _vp, _vp],
     "mb_sw_step_tile": [_M, ctypes.POINTER(MbFaceTiles), _P5, _P4, _d, _d, _i32, _i32, _vp, _vp, _vp, _vp, _vp],
     "mb_tet_tile_sizes": [_M, _i32, _vp, _vp, _vp],
     "mb_tet_tile_fill": [_M, ctypes.POINTER(MbTetTiles), _vp],

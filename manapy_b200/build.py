@@ -24,7 +24,7 @@ def nvcc():
 # the single-mesh and batched instantiations of one block body give identical bits.  The
 # Euler kernels likewise round every FP64 operation as manapy's (uncontracted) code does.
 FILE_FLAGS = {"fv_advdiff_f32c.cu": ["-fmad=false"], "fv_sw_f32c.cu": ["-fmad=false"],
-              "fv_euler.cu": ["-fmad=false"]}
+              "fv_euler.cu": ["-fmad=false"], "fv_euler_tile.cu": ["-fmad=false"]}
 
 
 def build(verbose=False, force=False):

@@ -16,50 +16,9 @@
 // every operation rounds as manapy's code does and the results are bit-identical to it.
 // manapy's flux reads the left cell's rhov in the right normal momentum
 // (qr = rhour n0 + rhovl n1); reproduced.
-#include "fv_common.cuh"
-#include "fv_compact.cuh"
+#include "fv_euler.cuh"
 
 namespace mb {
-
-struct EulerQ {
-  const double *rho, *P, *rhou, *rhov, *rhoE;
-};
-
-struct EulerW {
-  double *rho, *P, *rhou, *rhov, *rhoE;
-};
-
-__device__ __forceinline__ double dmax3(double a, double b, double c) {
-  // Python's max(a, b, c): the first of the largest
-  double m = a;
-  if (b > m) m = b;
-  if (c > m) m = c;
-  return m;
-}
-
-__device__ __forceinline__ void rusanov(double rhol, double Pl, double rhoul, double rhovl, double rhoEl, double rhor,
-                                        double Pr, double rhour, double rhovr, double rhoEr, double n0, double n1,
-                                        double mesure, double gamma, double F[4]) {
-  const double ql = (rhoul * n0 + rhovl * n1);
-  const double qr = (rhour * n0 + rhovl * n1);
-  const double cl = sqrt(gamma * Pl / rhol);
-  const double cr = sqrt(gamma * Pr / rhor);
-  const double fl_rho = (rhoul * n0 + rhovl * n1);
-  const double fl_rhou = ((rhoul * rhoul / rhol + Pl) * n0 + (rhoul * rhovl / rhol) * n1);
-  const double fl_rhov = ((rhovl * rhoul / rhol) * n0 + (rhovl * rhovl / rhol + Pl) * n1);
-  const double fl_rhoE = (rhoul / rhol * (rhoEl + Pl) * n0 + rhovl / rhol * (rhoEl + Pl) * n1);
-  const double fr_rho = (rhour * n0 + rhovr * n1);
-  const double fr_rhou = ((rhour * rhour / rhor + Pr) * n0 + (rhour * rhovr / rhor) * n1);
-  const double fr_rhov = ((rhovr * rhour / rhor) * n0 + (rhovr * rhovr / rhor + Pr) * n1);
-  const double fr_rhoE = (rhour / rhor * (rhoEr + Pr) * n0 + rhovr / rhor * (rhoEr + Pr) * n1);
-  const double Ll = dmax3(fabs(ql / rhol - cl), fabs(ql / rhol), fabs(ql / rhol + cl));
-  const double Lr = dmax3(fabs(qr / rhor - cr), fabs(qr / rhor), fabs(qr / rhor + cr));
-  const double S = Ll > Lr ? Ll : Lr;
-  F[0] = (0.5 * (fl_rho + fr_rho) - 0.5 * S * (rhor - rhol)) * mesure;
-  F[1] = (0.5 * (fl_rhou + fr_rhou) - 0.5 * S * (rhour - rhoul)) * mesure;
-  F[2] = (0.5 * (fl_rhov + fr_rhov) - 0.5 * S * (rhovr - rhovl)) * mesure;
-  F[3] = (0.5 * (fl_rhoE + fr_rhoE) - 0.5 * S * (rhoEr - rhoEl)) * mesure;
-}
 
 // the three faces of cell i in its own order (cells.faceid): ids, raw normals, measures
 __device__ __forceinline__ void cell_face_geom(const mb_mesh &m, int i, int f[3], double n0[3], double n1[3],
@@ -71,20 +30,6 @@ __device__ __forceinline__ void cell_face_geom(const mb_mesh &m, int i, int f[3]
     n1[j] = ld(m.face_normal + 3 * f[j] + 1);
     mes[j] = ld(m.face_mesure + f[j]);
   }
-}
-
-// time_step_euler_2d's per-cell dt, faces in the cell's own order
-__device__ __forceinline__ double euler_cell_dt(double rho, double P, double rhou, double rhov, const double n0[3],
-                                                const double n1[3], const double mes[3], double vol, double cfl,
-                                                double gamma) {
-  const double velson = sqrt(gamma * fabs(P / rho));
-  double lam = 0.;
-#pragma unroll
-  for (int j = 0; j < 3; ++j) {
-    const double u_n = fabs((rhou * n0[j] + rhov * n1[j]) / rho) / sqrt(n0[j] * n0[j] + n1[j] * n1[j]);
-    lam += (u_n + velson) * mes[j];
-  }
-  return cfl * vol / lam;
 }
 
 __global__ void __launch_bounds__(kBlock) k_euler_rusanov(mb_mesh m, EulerQ q, EulerQ g, double *r0, double *r1,
@@ -172,8 +117,6 @@ __global__ void __launch_bounds__(kBlock) k_ghost_euler_neumann(mb_mesh m, Euler
 // dt ring of three device slots: the step of time index t reads slot t%3 (the dt of its
 // input state, complete since the previous step), min-reduces the dt of its output state
 // into slot (t+1)%3, and resets slot (t+2)%3 for the step after.
-
-constexpr double kNoDt = 1e300;
 
 #ifndef MB_EULER_MIN_BLOCKS
 #define MB_EULER_MIN_BLOCKS 4

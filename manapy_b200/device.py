@@ -474,11 +474,15 @@ class DeviceMesh:
     FACE_TILE_CELLS = 256
     FACE_TILE_SLOTS = 740
 
+    # the Euler step keeps twice as much of a cell in shared memory (720,000 cells: 192 cells 56 us, 256
+    # 55, 320 68; 2M: 192 141, 256 169)
+    EULER_TILE_CELLS = 192
+
     @classmethod
-    def face_tile_cells(cls, nbcells):
-        nbcells = int(nbcells)
-        rounds = -(-nbcells // (cls.FACE_TILE_SLOTS * cls.FACE_TILE_CELLS))
-        return min(cls.FACE_TILE_CELLS, max(32, 16 * -(-nbcells // (16 * cls.FACE_TILE_SLOTS * rounds))))
+    def face_tile_cells(cls, nbcells, most=None):
+        nbcells, most = int(nbcells), cls.FACE_TILE_CELLS if most is None else int(most)
+        rounds = -(-nbcells // (cls.FACE_TILE_SLOTS * most))
+        return min(most, max(32, 16 * -(-nbcells // (16 * cls.FACE_TILE_SLOTS * rounds))))
 
     def _build_face_tiles(self, cells, stream):
         need = ("cell_vtx", "cell_xy", "cell_faces", "face_normal", "face_mesure", "cell_cellfid", "face_center",

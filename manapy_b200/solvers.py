@@ -1071,9 +1071,9 @@ class EulerSolver:
     One step composes them as: Neumann ghosts (``ghost_value_Neumann``, :592), residuals
     (``explicitscheme_euler_2d_rusanov``, :1490), ``dt`` = the min over cells of
     ``time_step_euler_2d`` (:1083), then ``update_euler_2d_fvc`` (:1687).
-    ``compute_new_val()`` / ``advance(n)`` run that step in two launches (every face flux once,
-    then update per cell), bit-identical to the sequence; the next step's ``dt`` is reduced on
-    the device in the update launch.  Every
+    ``compute_new_val()`` / ``advance(n)`` run that step in one launch on tiles of cells (every
+    face flux of a tile once in shared memory, then update per cell), bit-identical to the
+    sequence; the next step's ``dt`` is reduced on the device in the same launch.  Every
     boundary keeps the default Neumann rule.  ``compute_fluxes()`` leaves the residuals in
     ``var.convective`` (rho, rhou, rhov, rhoE) and the ghosts in ``var.ghost``, as the
     unfused kernels produce them.
@@ -1127,12 +1127,13 @@ class EulerSolver:
                           for _ in range(2)]
             self._ring = torch.full((3,), 1e300, dtype=f64, device=dm.device)
             self._time = torch.zeros(1, dtype=f64, device=dm.device)
-            self._ff = torch.empty(4 * dm.nbfaces, dtype=f64, device=dm.device)   # face fluxes
-            # static tables of the fused step: face records and left-cell bits
-            self._frec = torch.empty(4 * dm.nbfaces, dtype=f64, device=dm.device)
-            self._cleft = torch.empty(dm.nbcells, dtype=torch.uint8, device=dm.device)
-            _lib.call("mb_euler_tables_2d", dm.struct, _p(self._frec), _p(self._cleft),
-                      torch.cuda.current_stream(dm.device).cuda_stream)
+            self._tiles = dm.face_tiles(self._stream(), dm.face_tile_cells(dm.nbcells, dm.EULER_TILE_CELLS))
+            if self._tiles is None:
+                # the two-launch step: face fluxes, and its static tables (face records, left-cell bits)
+                self._ff = torch.empty(4 * dm.nbfaces, dtype=f64, device=dm.device)
+                self._frec = torch.empty(4 * dm.nbfaces, dtype=f64, device=dm.device)
+                self._cleft = torch.empty(dm.nbcells, dtype=torch.uint8, device=dm.device)
+                _lib.call("mb_euler_tables_2d", dm.struct, _p(self._frec), _p(self._cleft), self._stream())
             self._t = 0
             self._key = None
             self._dt_host = None
@@ -1201,6 +1202,11 @@ class EulerSolver:
     # ------------------------------------------------------------ fused step
     def _launch(self, t):
         a, b = self._bufs[t % 2], self._bufs[(t + 1) % 2]
+        if self._tiles is not None:
+            _lib.call("mb_euler_step_tile", self._dm.struct, self._tiles, _lib.p5([_p(x) for x in a]),
+                      _lib.p5([_p(x) for x in b]), self.cfl, self.gamma, _p(self._ring), int(t), _p(self._time),
+                      self._stream())
+            return
         _lib.call("mb_euler_step_2d", self._dm.struct, _lib.p5([_p(x) for x in a]), _lib.p5([_p(x) for x in b]),
                   self.cfl, self.gamma, _p(self._frec), _p(self._cleft), _p(self._ff), _p(self._ring), int(t),
                   _p(self._time), self._stream())
@@ -1257,4 +1263,4 @@ class EulerSolver:
         check_state([self.varbs[k].dev("cell") for k in self._NAMES], nonneg=(0, 1), names=list(self._NAMES))
 
     def launches_per_step(self):
-        return 2
+        return 2 if self._dm is None or self._tiles is None else 1
