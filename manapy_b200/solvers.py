@@ -67,7 +67,9 @@ class _Graphs:
         s.wait_stream(cur)
         g = torch.cuda.CUDAGraph()
         with torch.cuda.stream(s):
-            g.capture_begin()
+            # relaxed: what Python frees meanwhile (another solver's graph in a garbage collection, a
+            # thread's pinned buffer) must not invalidate the capture; the body only launches
+            g.capture_begin(capture_error_mode="relaxed")
             try:
                 body()
             finally:
@@ -1111,7 +1113,7 @@ class EulerSolver:
         self.dt = float(get("dt"))
         self.backend = self.domain.backend
         self._dm = None
-        self._graphs = {}
+        self._graphs = _Graphs()
 
     # ------------------------------------------------------------ state
     def _setup(self):
@@ -1237,14 +1239,10 @@ class EulerSolver:
             if graph and n >= D and self._t % 6 == 0:
                 g = self._graphs.get("main")
                 if g is None:
-                    s = torch.cuda.Stream(self._dm.device)
-                    s.wait_stream(torch.cuda.current_stream(self._dm.device))
-                    g = torch.cuda.CUDAGraph()
-                    with torch.cuda.graph(g, stream=s):
+                    def body():
                         for k in range(D):
                             self._launch(k)
-                    torch.cuda.current_stream(self._dm.device).wait_stream(s)
-                    self._graphs["main"] = g
+                    g = self._graphs.capture("main", self._dm.device, body)
                 g.replay()
                 self._t += D
                 n -= D
