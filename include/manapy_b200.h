@@ -472,6 +472,23 @@ int mb_advdiff_step_f32c(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_par
                          const float *sign_cf, const float *src, const double *dt_dev,
                          float *cell_scratch, float *node_scratch, void *stream);
 
+/* mb_advdiff_step_f32c with its coefficients in tables, bit-identical to it (tetrahedra at second order:
+ * to its step with the edge tables, which it needs).  mb_f32c_tables_fill forms them once for a mesh,
+ * order, diffusion coefficients and bc->face_grad_on, in FP64 rounded once: triangles geom
+ * [9][nbcells] (second order), coef [6][nbcells] (diffusion); tetrahedra coef [12][nbcells]; link [nbcells]; *status (device, zero before) becomes 1 where two
+ * cells share two faces (unsupported). */
+typedef struct mb_f32c_tables {
+  float *geom, *coef;
+  uint16_t *link;
+  int32_t *status;
+} mb_f32c_tables;
+int mb_f32c_tables_fill(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_params *p, const mb_f32c_tables *t,
+                        void *stream);
+int mb_advdiff_step_f32c_tab(const mb_mesh *m, const mb_f32c_tables *t, const mb_bc *bc, const mb_advdiff_params *p,
+                             const float *w_in, float *w_out, const float *lo_in, float *lo_out,
+                             const float *sign_cf, const float *src, const double *dt_dev, float *cell_scratch,
+                             float *node_scratch, void *stream);
+
 /* sign_cf[4*i+j] = u_face[f] n_x + v_face[f] n_y + w_face[f] n_z for the j-th local face f
  * of cell i (zero for unused slots): the upwind selector of
  * manapy/solvers/advecdiff/fvm_utils.py:53-64 laid out per cell for mb_advdiff_step */

@@ -74,6 +74,10 @@ class MbTetTables(ctypes.Structure):
     _fields_ = [("cell_q", _vp), ("link", _vp), ("node_mu", _vp), ("status", _vp)]
 
 
+class MbF32cTables(ctypes.Structure):
+    _fields_ = [("geom", _vp), ("coef", _vp), ("link", _vp), ("status", _vp)]
+
+
 class MbAdvDiffItem(ctypes.Structure):
     _fields_ = [("m", MbMesh), ("bc", MbBC), ("p", MbAdvDiffParams), ("w", _vp * 2), ("lo", _vp * 2), ("sign_cf", _vp),
                 ("src", _vp), ("dt_dev", _vp), ("cell_scratch", _vp), ("node_scratch", _vp),
@@ -183,6 +187,9 @@ _SIGS = {
     "mb_tet_tables_fill": [_M, ctypes.POINTER(MbTetTables), _vp],
     "mb_advdiff_step_tet_sums": [_M, ctypes.POINTER(MbTetTables), _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp,
                                  _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp],
+    "mb_f32c_tables_fill": [_M, _B, ctypes.POINTER(MbAdvDiffParams), ctypes.POINTER(MbF32cTables), _vp],
+    "mb_advdiff_step_f32c_tab": [_M, ctypes.POINTER(MbF32cTables), _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp,
+                                 _vp, _vp, _vp, _vp, _vp, _vp, _vp],
     "mb_tile_bytes": [ctypes.POINTER(MbTiles)],
     "mb_tile_coef": [_M, _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp],
     "mb_advdiff_step_tile": [_M, ctypes.POINTER(MbTiles), _B, ctypes.POINTER(MbAdvDiffParams), _vp, _vp, _vp, _vp,

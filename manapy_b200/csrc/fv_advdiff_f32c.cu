@@ -696,6 +696,8 @@ __global__ void __launch_bounds__(kBlock) k_f3c_sums(mb_mesh m, mb_bc bc, const 
 
 // cell pass: the gradient from the vertex, edge and face-neighbour sums (FP64, rounded once),
 // the Barth limiter in FP32 as k_f3c_phase1; the same records as k_f3c_phase1
+// FACES: records {e_0, .., e_3}, e_j = psi grad . (face centre - centre), for k_fc_flux
+template <bool FACES>
 __global__ void __launch_bounds__(kBlock, MB_P1C_3D_SUMS_MIN_BLOCKS)
     k_f3c_grad(mb_mesh m, mb_bc bc, const float *__restrict__ w, float *__restrict__ rec,
                const double *__restrict__ nrec, const double *__restrict__ erec) {
@@ -761,13 +763,14 @@ __global__ void __launch_bounds__(kBlock, MB_P1C_3D_SUMS_MIN_BLOCKS)
   const float gy = (float)((a1 * jx + a3 * jy + a4 * jz) * rdia);
   const float gz = (float)((a2 * jx + a4 * jy + a5 * jz) * rdia);
   const uint32_t fl = ld(m.cell_flags + i);
-  float ps = 1.f;
+  float ps = 1.f, de[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     int d0, d1, d2;
     face_desc(fl, j, d0, d1, d2);
     const D3 fc = (1. / 3) * tet_face_sum(P, j, d2);
     const float delta = gx * (float)(fc.x - c.x) + gy * (float)(fc.y - c.y) + gz * (float)(fc.z - c.z);
+    de[j] = delta;
     float psi_ij = 1.f;
     if (!(fabsf(delta) < 1e-10f)) {
       if (delta > 0.f) psi_ij = fminp(1.f, (wmax - wf) / delta);
@@ -776,8 +779,12 @@ __global__ void __launch_bounds__(kBlock, MB_P1C_3D_SUMS_MIN_BLOCKS)
     ps = fminp(ps, psi_ij);
   }
   const uint64_t keep = l2_keep();
-  st4_keep(rec + 4 * (long long)i, make_float4(wf, gx, gy, gz), keep);
-  st1f_keep(rec + 4 * (long long)m.nbcells + i, ps, keep);
+  if (FACES) {
+    st4_keep(rec + 4 * (long long)i, make_float4(ps * de[0], ps * de[1], ps * de[2], ps * de[3]), keep);
+  } else {
+    st4_keep(rec + 4 * (long long)i, make_float4(wf, gx, gy, gz), keep);
+    st1f_keep(rec + 4 * (long long)m.nbcells + i, ps, keep);
+  }
 }
 
 // FP32 u.n per cell face and, in FP64 then rounded, the cell's signed sum of them
@@ -800,6 +807,319 @@ __global__ void __launch_bounds__(kBlock) k_sign_f32c(mb_mesh m, const double *_
     s32[4 * (long long)m.nbcells + i] = (float)div;
 }
 
+// ---------------------------------------------------------------- steps with the geometry in tables
+//
+// The coefficients of the step depend on the mesh, the diffusion coefficients and the faces that
+// carry a gradient: formed once (mb_f32c_tables_fill) with the expressions of the kernels above, in
+// FP64 and rounded once, instead of by every step.  The first pass then stores what a face takes of
+// a cell, e_j = psi grad . (face centre - centre), and the second reads values and coefficients
+// only: no vertex, centre or normal.  The same operations on the same numbers, so the same bits.
+// What they were bound by is the latency of gathering geometry around every cell; B200, per step:
+// 2M triangles 180 -> 140, 500,000 43.8 -> 35.5 (first order 23.1 -> 17.4); 1.57M tetrahedra
+// 409 -> 353, 384,000 128 -> 116 (first order 41.7 -> 27.6).
+
+__device__ __forceinline__ unsigned f32c_link(const mb_mesh &m, int i) {
+  const int4 nb = ld4(m.cell_nbr + 4 * (long long)i);
+  const uint32_t fl = ld(m.cell_flags + i);
+  unsigned link = 0;
+  for (int j = 0; j < m.nlf; ++j) {
+    const int o = comp(nb, j);
+    link |= (m.dim == 2 ? (unsigned)f2_own(fl, j) : ((fl >> (6 * j)) & 1u)) << j;
+    if (o >= 0) {
+      const int4 back = ld4(m.cell_nbr + 4 * (long long)o);
+      link |= (unsigned)(back.x == i ? 0 : (back.y == i ? 1 : (back.z == i ? 2 : 3))) << (4 + 2 * j);
+    }
+  }
+  return link;
+}
+
+// triangles: geom planes a, b, e (inverse moment matrix) and the face centres' offsets; coef planes A_j, O_j
+__global__ void __launch_bounds__(kBlock) k_f2c_tables(mb_mesh m, mb_bc bc, mb_advdiff_params p, mb_f32c_tables t) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.nbcells) return;
+  const long long n = m.nbcells;
+  const double2 c = ldd2(m.cell_xy + 2 * (long long)i);
+  const int4 vt = ld4(m.cell_vtx + 4 * (long long)i), nb = ld4(m.cell_nbr + 4 * (long long)i);
+  const uint32_t fl = ld(m.cell_flags + i);
+  const double2 P0 = ldd2(m.node_coord + 2 * (long long)vt.x), P1 = ldd2(m.node_coord + 2 * (long long)vt.y),
+                P2 = ldd2(m.node_coord + 2 * (long long)vt.z);
+  t.link[i] = (uint16_t)f32c_link(m, i);
+  for (int j = 1; j < 3; ++j)     // the link's search for a face takes the neighbours as distinct
+    for (int q = 0; q < j; ++q)
+      if (comp(nb, j) >= 0 && comp(nb, j) == comp(nb, q)) atomicMax(t.status, 1);
+  if (p.order == 2) {
+    double ixx = 0., iyy = 0., ixy = 0.;
+    const int sb = ld(m.lsq_sell_ptr + (i >> 5)), se = ld(m.lsq_sell_ptr + (i >> 5) + 1);
+    for (int k = sb + (threadIdx.x & 31); k < se; k += 32) {
+      const int o = ld(m.lsq_sell_idx + k);
+      const double2 pc = ldd2(m.cell_xy + 2 * (long long)(o < 0 ? i : o));
+      const double dx = pc.x - c.x, dy = pc.y - c.y;
+      ixx += dx * dx; iyy += dy * dy; ixy += dx * dy;
+    }
+    for (int k = ld(m.ghostnid_ptr + i); k < ld(m.ghostnid_ptr + i + 1); ++k) {
+      const long long f = ld(m.ghostnid_idx + k);
+      const double dx = ld(m.face_ghostcenter + 3 * f) - c.x, dy = ld(m.face_ghostcenter + 3 * f + 1) - c.y;
+      ixx += dx * dx; iyy += dy * dy; ixy += dx * dy;
+    }
+    const double rdia = 1. / (ixx * iyy - ixy * ixy);
+    t.geom[i] = (float)(iyy * rdia);
+    t.geom[n + i] = (float)(ixy * rdia);
+    t.geom[2 * n + i] = (float)(ixx * rdia);
+  }
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const double2 Pj = j == 0 ? P0 : (j == 1 ? P1 : P2), Pk = j == 0 ? P1 : (j == 1 ? P2 : P0);
+    if (p.order == 2) {
+      t.geom[(3 + 2 * j) * n + i] = (float)(0.5 * (Pj.x + Pk.x) - c.x);
+      t.geom[(4 + 2 * j) * n + i] = (float)(0.5 * (Pj.y + Pk.y) - c.y);
+    }
+    if (!p.diffusion) continue;
+    const int o = comp(nb, j), f = -1 - o;
+    float A = 0.f, O = 0.f;
+    if (o >= 0 || ld(bc.face_grad_on + f)) {
+      const bool own = f2_own(fl, j), rev = f2_rev(fl, j);
+      const double2 Xa = rev ? Pk : Pj, Xb = rev ? Pj : Pk;
+      const double2 co = o < 0 ? make_double2(ld(m.face_ghostcenter + 3 * (long long)f),
+                                              ld(m.face_ghostcenter + 3 * (long long)f + 1))
+                               : ldd2(m.cell_xy + 2 * (long long)o);
+      const double2 v1 = own ? c : co, v2 = own ? co : c;
+      const double air = 0.5 * ((Xb.x - Xa.x) * (v2.y - v1.y) + (v1.x - v2.x) * (Xb.y - Xa.y));
+      double n0 = Xa.y - Xb.y, n1 = Xb.x - Xa.x;
+      if (f2_flip(fl, j)) { n0 = -1 * n0; n1 = -1 * n1; }
+      const double r2a = 1. / (2 * air);
+      const double gxk = p.Dxx * n0 * r2a, gyk = p.Dyy * n1 * r2a;
+      const double a1 = gxk * (v1.y - v2.y) - gyk * (v1.x - v2.x);
+      const double al = gxk * (Xb.y - Xa.y) - gyk * (Xb.x - Xa.x);
+      // signs (side of the face, order of its vertices) are exact
+      A = own != rev ? (float)a1 : -(float)a1;
+      O = (float)-al;
+    }
+    t.coef[j * n + i] = A;
+    t.coef[(3 + j) * n + i] = O;
+  }
+}
+
+// first pass: records {w, e_0, e_1, e_2}; node blocks as k_f2c_phase1
+// 8 blocks per SM (32 registers): 500,000 triangles 35.5 us per step, 6 blocks 37.9; with the centre
+// offsets of every slot read from a table instead of subtracting gathered centres 42.4
+#ifndef MB_F2C_CELLS_MIN
+#define MB_F2C_CELLS_MIN 8
+#endif
+template <bool DIFF>
+__global__ void __launch_bounds__(kBlock, MB_F2C_CELLS_MIN) k_f2c_cells(mb_mesh m, mb_f32c_tables t, mb_bc bc,
+                                                         const float *__restrict__ w, float *__restrict__ rec,
+                                                         float *__restrict__ wn, int ncb) {
+  const GhostRuleF ghost = make_rule_f(m, bc, w);
+  const int lane = threadIdx.x & 31;
+  if ((int)blockIdx.x >= ncb) {
+    if (DIFF) node_value_f32(m, ghost, w, wn, ((int)blockIdx.x - ncb) * blockDim.x + threadIdx.x, lane);
+    return;
+  }
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.nbcells) return;
+  const long long n = m.nbcells;
+  const float wi = ld(w + i);
+  const double2 c = ldd2(m.cell_xy + 2 * (long long)i);
+  float jx = 0.f, jy = 0.f;
+  const int sb = ld(m.lsq_sell_ptr + (i >> 5)) + lane, L = (ld(m.lsq_sell_ptr + (i >> 5) + 1) - (sb - lane)) >> 5;
+  const uint64_t pst = l2_stream();
+  for (int k = 0; k < L; k += 4) {
+    int o[4];
+    float2 d[4];
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      o[u] = k + u < L ? ld1_stream(m.lsq_sell_idx + sb + 32 * (k + u), pst) : -1;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const double2 pc = o[u] < 0 ? c : ldd2(m.cell_xy + 2 * (long long)o[u]);
+      d[u] = make_float2((float)(pc.x - c.x), (float)(pc.y - c.y));
+      v[u] = o[u] < 0 ? wi : ld(w + o[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float dw = v[u] - wi;
+      jx = fmaf(d[u].x, dw, jx);
+      jy = fmaf(d[u].y, dw, jy);
+    }
+  }
+  const int gb = ld(m.ghostnid_ptr + i), ge = ld(m.ghostnid_ptr + i + 1);
+  for (int k = gb; k < ge; ++k) {
+    const int f = ld(m.ghostnid_idx + k);
+    const double dx = ld(m.face_ghostcenter + 3 * (long long)f) - c.x,
+                 dy = ld(m.face_ghostcenter + 3 * (long long)f + 1) - c.y;
+    const float dw = ghost(f) - wi;
+    jx = fmaf((float)dx, dw, jx); jy = fmaf((float)dy, dw, jy);
+  }
+  const float a = ldf_stream(t.geom + i, pst), b = ldf_stream(t.geom + n + i, pst),
+              e = ldf_stream(t.geom + 2 * n + i, pst);
+  const float x = a * jx - b * jy;
+  const float y = e * jy - b * jx;
+  const int4 nb = ld4(m.cell_nbr + 4 * (long long)i);
+  float wmax = wi, wmin = wi;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const int o = comp(nb, j);
+    const float bv = o < 0 ? ghost(-1 - o) : ld(w + o);
+    wmax = fmaxp(wmax, bv);
+    wmin = fminp(wmin, bv);
+  }
+  float ps = 1.f, delta[3];
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    const float r1 = ldf_stream(t.geom + (3 + 2 * j) * n + i, pst), r2 = ldf_stream(t.geom + (4 + 2 * j) * n + i, pst);
+    delta[j] = x * r1 + y * r2;
+    float psi_ij = 1.f;
+    if (!(fabsf(delta[j]) < 1e-8f)) {
+      if (delta[j] > 0.f) psi_ij = fminp(1.f, (wmax - wi) / delta[j]);
+      if (delta[j] < 0.f) psi_ij = fminp(1.f, (wmin - wi) / delta[j]);
+    }
+    ps = fminp(ps, psi_ij);
+  }
+  st4_keep(rec + 4 * (long long)i, make_float4(wi, ps * delta[0], ps * delta[1], ps * delta[2]), l2_keep());
+}
+
+// second pass of a cell with NF faces: fluxes of the recorded values and the update.  DIM 2: rec
+// {w, e_0, e_1, e_2}; DIM 3: rec {e_0, .., e_3} and the state itself
+template <int DIM, bool ORDER2, bool DIFF>
+__global__ void __launch_bounds__(128, 8)
+    k_fc_flux(mb_mesh m, mb_f32c_tables t, mb_bc bc, const float *__restrict__ w, float *__restrict__ w_out,
+              const float *__restrict__ sign, const float *__restrict__ src, const double *__restrict__ dt_dev,
+              const float *__restrict__ rec, const float *__restrict__ wn, const float *__restrict__ lo_in,
+              float *__restrict__ lo_out) {
+  constexpr int NF = DIM == 2 ? 3 : 4;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.nbcells) return;
+  const GhostRuleF ghost = make_rule_f(m, bc, w);
+  const long long n = m.nbcells;
+  const uint64_t pst = l2_stream();
+  const int4 nb = ld4(m.cell_nbr + 4 * (long long)i);
+  const unsigned link = ld(t.link + i);
+  const float4 s4 = ldf4(sign + 4 * (long long)i);
+  const float s[4] = {s4.x, s4.y, s4.z, s4.w};
+  float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (ORDER2) r = ldf4(rec + 4 * (long long)i);
+  const float wi = ORDER2 && DIM == 2 ? r.x : ld(w + i);
+  const float mine[4] = {DIM == 2 ? r.y : r.x, DIM == 2 ? r.z : r.y, DIM == 2 ? r.w : r.z, r.w};
+  float cv[4], q[4], dv[4];
+#pragma unroll
+  for (int j = 0; j < NF; ++j) {
+    const int o = comp(nb, j);
+    const bool b = o < 0, own = (link >> j) & 1u;
+    const int peer = (link >> (4 + 2 * j)) & 3u;
+    const bool take_me = (s[j] >= 0.f) == own;
+    float vo, far = 0.f;
+    if (b) {
+      vo = ghost(-1 - o);
+    } else if (ORDER2 && DIM == 2) {
+      const float4 x = ldf4(rec + 4 * (long long)o);
+      vo = x.x;
+      far = peer == 0 ? x.y : (peer == 1 ? x.z : x.w);
+    } else {
+      vo = ld(w + o);
+      if (ORDER2 && !take_me) far = ld(rec + 4 * (long long)o + peer);
+    }
+    dv[j] = vo - wi;
+    float dsol;
+    if (take_me) dsol = ORDER2 ? mine[j] : 0.f;
+    else if (b) dsol = dv[j];
+    else dsol = ORDER2 ? dv[j] + far : dv[j];
+    const float F = s[j] * dsol;
+    cv[j] = own ? -F : F;
+    q[j] = 0.f;
+  }
+  if (DIFF) {
+    const int4 vt = ld4(m.cell_vtx + 4 * (long long)i);
+    const float v[4] = {ld(wn + vt.x), ld(wn + vt.y), ld(wn + vt.z), DIM == 3 ? ld(wn + vt.w) : 0.f};
+    const uint32_t fl = DIM == 3 ? ld(m.cell_flags + i) : 0u;
+#pragma unroll
+    for (int j = 0; j < NF; ++j) {
+      if (DIM == 2) {
+        const float A = ldf_stream(t.coef + j * n + i, pst), O = ldf_stream(t.coef + (3 + j) * n + i, pst);
+        if (O != 0.f) q[j] = A * (v[j] - v[(j + 1) % 3]) + O * dv[j];   // 0: a face without a gradient
+      } else {
+        const float ca = ldf_stream(t.coef + (3 * j) * n + i, pst), cb = ldf_stream(t.coef + (3 * j + 1) * n + i, pst),
+                    cr = ldf_stream(t.coef + (3 * j + 2) * n + i, pst);
+        int d0, d1, d2;
+        face_desc(fl, j, d0, d1, d2);
+        const bool swp = (fl >> (6 * j + 4)) & 1u;
+        const float VA = pick4v(v[0], v[1], v[2], v[3], d0), VB = pick4v(v[0], v[1], v[2], v[3], swp ? d2 : d1),
+                    VC = pick4v(v[0], v[1], v[2], v[3], swp ? d1 : d2);
+        if (cr != 0.f) q[j] = ca * (VA - VC) + cb * (VB - VC) + cr * dv[j];
+      }
+    }
+  }
+  const uint8_t code = ld(m.cell_order + i);
+  auto at = [&](const float *x, int sl) {
+    return DIM == 2 ? pick3(x[0], x[1], x[2], sl) : pick4v(x[0], x[1], x[2], x[3], sl);
+  };
+  CompSum res;
+#pragma unroll
+  for (int k = 0; k < NF; ++k) {
+    const int sl = order_slot(code, k);
+    if ((DIM == 2 ? pick3(nb.x, nb.y, nb.z, sl) : pick4v(nb.x, nb.y, nb.z, nb.w, sl)) >= 0) res.add(at(cv, sl));
+  }
+#pragma unroll
+  for (int k = 0; k < NF; ++k) {
+    const int sl = order_slot(code, k);
+    if ((DIM == 2 ? pick3(nb.x, nb.y, nb.z, sl) : pick4v(nb.x, nb.y, nb.z, nb.w, sl)) < 0) res.add(at(cv, sl));
+  }
+  res.add(wi * (DIM == 2 ? s4.w : ld(sign + 4 * n + i)));  // w_i times the cell's signed u.n sum
+  if (DIFF) {
+#pragma unroll
+    for (int k = 0; k < NF; ++k) res.add(at(q, order_slot(code, k)));
+  }
+  const double dt = *dt_dev;
+  float inc = (float)(dt / ld(m.cell_volume + i)) * res.value();
+  if (src) inc = fmaf((float)dt, ld(src + i), inc);
+  store_state(wi, inc, lo_in, w_out, lo_out, i);
+}
+
+// tetrahedra: coef planes ca, cb, cr of every face
+__global__ void __launch_bounds__(kBlock) k_f3c_tables(mb_mesh m, mb_bc bc, mb_advdiff_params p, mb_f32c_tables t) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= m.nbcells) return;
+  const long long n = m.nbcells;
+  const int4 vt = ld4(m.cell_vtx + 4 * (long long)i), nb = ld4(m.cell_nbr + 4 * (long long)i);
+  const uint32_t fl = ld(m.cell_flags + i);
+  const D3 ci = ld3(m.cell_xy + 4 * (long long)i);
+  t.link[i] = (uint16_t)f32c_link(m, i);
+  for (int j = 1; j < 4; ++j)
+    for (int q = 0; q < j; ++q)
+      if (comp(nb, j) >= 0 && comp(nb, j) == comp(nb, q)) atomicMax(t.status, 1);
+  if (!p.diffusion) return;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const int o = comp(nb, j), f = -1 - o;
+    float ca = 0.f, cb = 0.f, cr = 0.f;
+    if (o >= 0 || ld(bc.face_grad_on + f)) {
+      const bool own = (fl >> (6 * j)) & 1u;
+      int d0, d1, d2;
+      face_desc(fl, j, d0, d1, d2);
+      const D3 V0 = ld3(m.node_coord + 4 * (long long)comp(vt, d0)), V1 = ld3(m.node_coord + 4 * (long long)comp(vt, d1)),
+               V2 = ld3(m.node_coord + 4 * (long long)comp(vt, d2));
+      const double *gc = m.face_ghostcenter + 3 * (long long)(o < 0 ? f : 0);
+      const D3 co = o < 0 ? d3(ld(gc), ld(gc + 1), ld(gc + 2)) : ld3(m.cell_xy + 4 * (long long)o);
+      const D3 Nd = 0.5 * cross(V1 - V0, V2 - V0);
+      const D3 N = ((fl >> (6 * j + 5)) & 1u) ? (-1.0) * Nd : Nd;
+      const bool swp = (fl >> (6 * j + 4)) & 1u;
+      const D3 Q2 = swp ? V2 : V1, Q3 = swp ? V1 : V2;
+      const D3 v1 = own ? ci : co, v2 = own ? co : ci;
+      const double rair = 1. / dot(N, v2 - v1);
+      const D3 DN = d3(p.Dxx * N.x, p.Dyy * N.y, p.Dzz * N.z);
+      const D3 tt = cross(v1 - v2, DN);
+      ca = (float)(0.5 * dot(Q3 - Q2, tt) * rair);
+      cb = (float)(0.5 * dot(V0 - Q3, tt) * rair);
+      cr = (float)(dot(DN, N) * rair);
+      if (!own) { ca = -ca; cb = -cb; }     // the flux leaves the other way; cr's difference turns too
+    }
+    t.coef[(3 * j) * n + i] = ca;
+    t.coef[(3 * j + 1) * n + i] = cb;
+    t.coef[(3 * j + 2) * n + i] = cr;
+  }
+}
+
 template <bool O2, bool DF>
 int launch_step_f32c(const mb_mesh &m, const mb_bc &bc, const mb_advdiff_params &p, const float *w_in, float *w_out,
                      const float *sign, const float *src, const double *dt, float *cs, float *wn, const float *lo_in,
@@ -818,7 +1138,7 @@ int launch_step_f32c(const mb_mesh &m, const mb_bc &bc, const mb_advdiff_params 
       double *nrec = reinterpret_cast<double *>(cs + f3c_rec_floats(m)), *erec = nrec + 4 * (long long)m.nbnodes;
       const int nvb = ceil_div(m.nbnodes, kBlock), neb = ceil_div(m.nbedges, kBlock);
       k_f3c_sums<DF><<<nvb + neb, kBlock, 0, st>>>(m, bc, w_in, nrec, erec, wn, nvb);
-      k_f3c_grad<<<ceil_div(m.nbcells, kBlock), kBlock, 0, st>>>(m, bc, w_in, cs, nrec, erec);
+      k_f3c_grad<false><<<ceil_div(m.nbcells, kBlock), kBlock, 0, st>>>(m, bc, w_in, cs, nrec, erec);
     } else if (ncb + nnb > 0) {
       if (O2 && m.cell_lsq)
         k_f3c_phase1<O2, DF, true><<<ncb + nnb, kBlock, 0, st>>>(m, bc, w_in, cs, wn, ncb);
@@ -831,9 +1151,81 @@ int launch_step_f32c(const mb_mesh &m, const mb_bc &bc, const mb_advdiff_params 
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
 }
 
+template <bool O2, bool DF>
+int launch_step_f32c_tab(const mb_mesh &m, const mb_f32c_tables &t, const mb_bc &bc, const float *w_in, float *w_out,
+                         const float *sign, const float *src, const double *dt, float *cs, float *wn,
+                         const float *lo_in, float *lo_out, cudaStream_t st) {
+  const int ncb = ceil_div(m.nbcells, kBlock), nnb = DF ? ceil_div(m.nbnodes, kBlock) : 0;
+  const int fb = ceil_div(m.nbcells, 128);
+  if (m.dim == 2) {
+    if (O2) k_f2c_cells<DF><<<ncb + nnb, kBlock, 0, st>>>(m, t, bc, w_in, cs, wn, ncb);
+    else if (DF) k_f2c_phase1<false, true><<<nnb, kBlock, 0, st>>>(m, bc, w_in, cs, wn, 0);
+    k_fc_flux<2, O2, DF><<<fb, 128, 0, st>>>(m, t, bc, w_in, w_out, sign, src, dt, cs, wn, lo_in, lo_out);
+  } else {
+    if (O2) {
+      if (!f3c_sums_tables(m) || (reinterpret_cast<uintptr_t>(cs) & 31) != 0 ||
+          (reinterpret_cast<uintptr_t>(m.cell_lsq) & 31) != 0)
+        return MB_EINVAL;
+      double *nrec = reinterpret_cast<double *>(cs + f3c_rec_floats(m)), *erec = nrec + 4 * (long long)m.nbnodes;
+      const int nvb = ceil_div(m.nbnodes, kBlock), neb = ceil_div(m.nbedges, kBlock);
+      k_f3c_sums<DF><<<nvb + neb, kBlock, 0, st>>>(m, bc, w_in, nrec, erec, wn, nvb);
+      k_f3c_grad<true><<<ncb, kBlock, 0, st>>>(m, bc, w_in, cs, nrec, erec);
+    } else if (DF) {
+      k_f3c_phase1<false, true, false><<<nnb, kBlock, 0, st>>>(m, bc, w_in, cs, wn, 0);
+    }
+    k_fc_flux<3, O2, DF><<<fb, 128, 0, st>>>(m, t, bc, w_in, w_out, sign, src, dt, cs, wn, lo_in, lo_out);
+  }
+  return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
+}
+
 }  // namespace mb
 
 using namespace mb;
+
+extern "C" int mb_f32c_tables_fill(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_params *p,
+                                   const mb_f32c_tables *t, void *stream) {
+  MB_NVTX();
+  if (!m || (m->dim != 2 && m->dim != 3) || m->nbcells <= 0 || !bc || !p || (p->order != 1 && p->order != 2) || !t ||
+      !t->link || !t->status || (p->diffusion && (!t->coef || !bc->face_grad_on)) ||
+      (m->dim == 2 && p->order == 2 && (!t->geom || !m->lsq_sell_ptr || !m->lsq_sell_idx)))
+    return MB_EINVAL;
+  if (!m->cell_vtx || !m->cell_nbr || !m->cell_flags || !m->node_coord || !m->cell_xy || !m->ghostnid_ptr ||
+      !m->ghostnid_idx || !m->face_ghostcenter ||
+      (m->dim == 3 && (((uintptr_t)m->cell_xy | (uintptr_t)m->node_coord) & 31)))
+    return MB_EINVAL;
+  const int b = ceil_div(m->nbcells, kBlock);
+  if (m->dim == 2) k_f2c_tables<<<b, kBlock, 0, (cudaStream_t)stream>>>(*m, *bc, *p, *t);
+  else k_f3c_tables<<<b, kBlock, 0, (cudaStream_t)stream>>>(*m, *bc, *p, *t);
+  return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
+}
+
+extern "C" int mb_advdiff_step_f32c_tab(const mb_mesh *m, const mb_f32c_tables *t, const mb_bc *bc,
+                                        const mb_advdiff_params *p, const float *w_in, float *w_out,
+                                        const float *lo_in, float *lo_out, const float *sign_cf, const float *src,
+                                        const double *dt_dev, float *cell_scratch, float *node_scratch, void *stream) {
+  MB_NVTX();
+  if (!m || !t || !bc || !p || !w_in || !w_out || !sign_cf || !dt_dev || w_in == w_out) return MB_EINVAL;
+  if ((m->dim != 2 && m->dim != 3) || m->nbcells <= 0 || (p->order != 1 && p->order != 2)) return MB_EINVAL;
+  if ((lo_in == nullptr) != (lo_out == nullptr) || (lo_in && lo_in == lo_out)) return MB_EINVAL;
+  const bool o2 = p->order == 2, df = p->diffusion != 0;
+  if (!m->cell_vtx || !m->cell_nbr || !m->cell_flags || !m->cell_order || !m->cell_volume || !m->node_coord ||
+      !m->cell_xy || !m->lsq_sell_ptr || !m->lsq_sell_idx || !m->n2c_sell_ptr || !m->n2c_sell_idx ||
+      !m->n2c_sell_alpha_f32 || !t->link || !bc->kind || !bc->value)
+    return MB_EINVAL;
+  if ((o2 && !cell_scratch) || (df && (!node_scratch || !t->coef)) || (o2 && m->dim == 2 && !t->geom) ||
+      (((uintptr_t)cell_scratch | (uintptr_t)sign_cf) & 15) ||
+      (m->dim == 3 && (((uintptr_t)m->cell_xy | (uintptr_t)m->node_coord) & 31)))
+    return MB_EINVAL;
+  cudaStream_t st = (cudaStream_t)stream;
+#define MB_F32C(O, D)                                                                                               \
+  return launch_step_f32c_tab<O, D>(*m, *t, *bc, w_in, w_out, sign_cf, src, dt_dev, cell_scratch, node_scratch, lo_in, \
+                                    lo_out, st)
+  if (o2 && df) MB_F32C(true, true);
+  if (o2) MB_F32C(true, false);
+  if (df) MB_F32C(false, true);
+  MB_F32C(false, false);
+#undef MB_F32C
+}
 
 extern "C" int mb_advdiff_step_f32c(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_params *p,
                                     const float *w_in, float *w_out, const float *lo_in, float *lo_out,

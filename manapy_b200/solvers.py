@@ -433,6 +433,7 @@ class AdvectionDiffusionSolver:
             self._ns32 = torch.empty(dm.nbnodes, dtype=torch.float32, device=dm.device)
             self._sign32 = torch.empty((4 if dm.dim == 2 else 5) * dm.nbcells, dtype=torch.float32,
                                        device=dm.device)
+            self._f32_tables()
         if var.version("cell") != self._w32_key:
             w64 = var.dev("cell")
             hi = self._w32[self._w32_i]
@@ -440,6 +441,29 @@ class AdvectionDiffusionSolver:
             self._lo32[self._w32_i].copy_(w64 - hi.double())
             self._w32_key = var.version("cell")
         return self._w32[self._w32_i]
+
+    def _f32_tables(self):
+        """The FP32 step's coefficients (``_lib.MbF32cTables``), formed once; None where the step forms
+        them itself (tetrahedra at second order without the edge sums, or a missing table)."""
+        dm = self._dm
+        self._tab32 = None
+        need = ("cell_vtx", "ghostnid_ptr", "face_ghostcenter", "lsq_sell_idx", "n2c_sell_alpha_f32")
+        if any(n not in dm.t for n in need) or \
+                (dm.dim == 3 and self.order == 2 and not (dm.struct.cell_edges and dm.struct.n2c_sum_ptr)):
+            return
+        n, f = dm.nbcells, 4
+        sizes = {"link": 2 * n}
+        if self.diffusion:
+            sizes["coef"] = f * (6 if dm.dim == 2 else 12) * n
+        if dm.dim == 2 and self.order == 2:
+            sizes["geom"] = f * 9 * n
+        t = _lib.MbF32cTables()
+        buf = dm._carve(t, sizes)
+        status = torch.zeros(1, dtype=torch.int32, device=dm.device)
+        t.status = _p(status)
+        _lib.call("mb_f32c_tables_fill", dm.struct, self.var.device_bc.struct, self._params, t, self._stream())
+        if not int(status.item()):
+            self._tab32, self._tab32_keep = t, (buf, status)
 
     def _f64_of(self, k):
         """FP64 value of FP32 state buffer ``k`` (w + lo)."""
@@ -480,9 +504,11 @@ class AdvectionDiffusionSolver:
             # another solver on this mesh opted its struct into the edge sums since the
             # scratch was sized
             self._cs32 = torch.empty(self._dm.cell_scratch_size_f32c(), dtype=torch.float32, device=self._dm.device)
-        _lib.call("mb_advdiff_step_f32c", self._dm.struct, self.var.device_bc.struct, self._params, _p(w[k]),
-                  _p(w[1 - k]), _p(lo[k]), _p(lo[1 - k]), _p(self._sign32), _p(src), _p(self._dt_dev),
-                  _p(self._cs32), _p(self._ns32), st)
+        name, tab = ("mb_advdiff_step_f32c", ()) if self._tab32 is None else \
+            ("mb_advdiff_step_f32c_tab", (self._tab32,))
+        _lib.call(name, self._dm.struct, *tab, self.var.device_bc.struct, self._params, _p(w[k]), _p(w[1 - k]),
+                  _p(lo[k]), _p(lo[1 - k]), _p(self._sign32), _p(src), _p(self._dt_dev), _p(self._cs32),
+                  _p(self._ns32), st)
 
     def _fused_step_f32c(self):
         self._f32_state()
