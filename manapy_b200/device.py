@@ -420,8 +420,7 @@ class DeviceMesh:
             self._tiles = {}
         if cells not in self._tiles:
             self._tiles[cells] = self._build_tiles(cells, stream)
-        got = self._tiles[cells]
-        return None if got is None else got[0]
+        return self._tiles[cells]
 
     def _build_tiles(self, cells, stream):
         need = ("cell_vtx", "cell_xy", "n2c_ptr", "n2c_alpha", "n2g_ptr", "n2g_alpha", "lsq_sell_idx", "ghostnid_ptr",
@@ -454,7 +453,7 @@ class DeviceMesh:
         buf = self._carve(t, sizes, head)
         scratch = torch.empty(4 * (self.nbcells + self.nbnodes), dtype=torch.float64, device=dev)
         _lib.call("mb_tile_fill", self.struct, t, scratch.data_ptr(), st)
-        return t, (head, buf)
+        return self._filled(t, head, buf, st)
 
     def face_tiles(self, stream=None, cells=None):
         """The tiles of a triangle mesh with their faces (``_lib.MbFaceTiles``), built on the device on
@@ -465,8 +464,7 @@ class DeviceMesh:
             self._face_tiles = {}
         if cells not in self._face_tiles:
             self._face_tiles[cells] = self._build_face_tiles(cells, stream)
-        got = self._face_tiles[cells]
-        return None if got is None else got[0]
+        return self._face_tiles[cells]
 
     # a B200 runs 148 SMs x 5 blocks of that kernel at once; with larger tiles fewer blocks fit an
     # SM's shared memory (1.28M cells: 256 cells 80 us, 288 93).  One round of blocks where the mesh
@@ -502,11 +500,12 @@ class DeviceMesh:
         up = lambda n, k: -(-n // k) * k  # noqa: E731
         t = _lib.MbFaceTiles()
         t.cells, t.count, t.out_cap, t.face_cap = cells, count, out, up(faces, 4)
-        return t, (head, self._carve(t, {"out": 4 * count * out, "face": 4 * count * t.face_cap,
-                                         "face_n0": 8 * count * t.face_cap, "face_n1": 8 * count * t.face_cap,
-                                         "face_mes": 8 * count * t.face_cap, "cell": 16 * count * cells,
-                                         "cell_ns": 16 * self.nbcells}, head),
-                   _lib.call("mb_face_tile_fill", self.struct, t, st))
+        buf = self._carve(t, {"out": 4 * count * out, "face": 4 * count * t.face_cap,
+                              "face_n0": 8 * count * t.face_cap, "face_n1": 8 * count * t.face_cap,
+                              "face_mes": 8 * count * t.face_cap, "cell": 16 * count * cells,
+                              "cell_ns": 16 * self.nbcells}, head)
+        _lib.call("mb_face_tile_fill", self.struct, t, st)
+        return self._filled(t, head, buf, st)
 
     # Tetrahedra, second order (fv_tet_tile.cu): a B200 runs 148 SMs x 2 blocks of the tiled gradient pass
     # at once; tiles of one or two rounds of blocks, at most 256 cells (shared memory).  A tile has
@@ -531,8 +530,7 @@ class DeviceMesh:
             self._tet_tiles = {}
         if cells not in self._tet_tiles:
             self._tet_tiles[cells] = self._build_tet_tiles(cells, stream)
-        got = self._tet_tiles[cells]
-        return None if got is None else got[0]
+        return self._tet_tiles[cells]
 
     def _build_tet_tiles(self, cells, stream):
         need = ("cell_vtx", "cell_xy", "n2c_ptr", "n2c_alpha", "n2g_ptr", "ghostnid_ptr", "face_ghostcenter", "cell_lsq",
@@ -565,7 +563,7 @@ class DeviceMesh:
                               "ninc": 2 * count * t.ninc_cap, "einc": 2 * count * t.einc_cap, "cell": 32 * nc,
                               "cell_q": 96 * nc, "link": 2 * nc}, head)
         _lib.call("mb_tet_tile_fill", self.struct, t, st)
-        return t, (head, buf)
+        return self._filled(t, head, buf, st)
 
     def tet_tables(self, stream=None):
         """The tables of the second-order step on large tetrahedral meshes (``_lib.MbTetTables``), built on
@@ -574,7 +572,7 @@ class DeviceMesh:
         if getattr(self, "_tet_tables", None) is None:
             need = ("cell_lsq", "cell_edges", "edge_sell_idx", "n2c_sum_idx", "n2c_ptr", "n2c_alpha", "n2g_ptr",
                     "ghostnid_ptr", "face_ghostcenter")
-            self._tet_tables = (None, None)
+            got = False
             if self.dim == 3 and self.device is not None and self.stencil == "shared" and \
                     all(n in self.t for n in need):
                 nc, nn = self.nbcells, self.nbnodes
@@ -585,8 +583,17 @@ class DeviceMesh:
                 st = stream if stream is not None else torch.cuda.current_stream(self.device).cuda_stream
                 _lib.call("mb_tet_tables_fill", self.struct, t, st)
                 if not int(status.item()):
-                    self._tet_tables = (t, (buf, status))
-        return self._tet_tables[0]
+                    got = self._filled(t, status, buf, st)
+            self._tet_tables = got
+        return self._tet_tables or None
+
+    def _filled(self, t, head, buf, st):
+        """``t`` with the memory that its pointers name, once its tables are there: solvers on other
+        streams share them, and may outlive this mesh."""
+        (torch.cuda.ExternalStream(st, device=self.device) if st else
+         torch.cuda.default_stream(self.device)).synchronize()
+        t.memory = (head, buf)
+        return t
 
     def _carve(self, t, sizes, head=None):
         """One device allocation for the tables of ``t`` (bytes by field), at 256-byte boundaries."""

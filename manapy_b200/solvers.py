@@ -377,6 +377,11 @@ class AdvectionDiffusionSolver:
             self._rows_version = self.var.version("cell")
         return self._rows_of(buf)
 
+    def _on_tiles(self, w):
+        """Whether a step from cell array ``w`` runs on tiles: the triangles' copies ``w`` in 16-byte
+        pieces, so an array installed at an odd offset of its storage takes the two-launch step."""
+        return self._tiles is not None and (self.dim == 3 or w.data_ptr() % 16 == 0)
+
     def _call_step(self, w_in, w_out, src, st):
         """The kernels of one FP64 step (the rows of ``w_in`` current where they are used)."""
         dm, bc = self._dm, self.var.device_bc.struct
@@ -391,7 +396,7 @@ class AdvectionDiffusionSolver:
                       _p(self._rows_of(w_in)), _p(self._rows_of(w_out)), _p(self._sign), _p(self._coef), src,
                       _p(self._dt_dev), _p(cs), _p(ns), st)
             return
-        if self._tiles is not None:
+        if self._on_tiles(w_in):
             _lib.call("mb_advdiff_step_tile", dm.struct, self._tiles, bc, self._params, _p(w_in), _p(w_out),
                       _p(self._sign), _p(self._coef), src, _p(self._dt_dev), st)
             return
@@ -645,7 +650,7 @@ class AdvectionDiffusionSolver:
         if self._graph_bufs is None:
             self._graph_bufs = (var.dev("cell"), self._spare)
         a, b = self._graph_bufs
-        if self._tiles is None or self.dim == 3:
+        if self.dim == 3 or not (self._on_tiles(a) and self._on_tiles(b)):
             self._scratch()             # allocated before the capture
         if self._use_rows():
             self._rows_of(a), self._rows_of(b)
@@ -808,6 +813,11 @@ class ShallowWaterSolver:
     def _q(self):
         return [self.varbs[k].dev("cell") for k in ("h", "hu", "hv", "hc", "Z")]
 
+    def _on_tiles(self, q):
+        """Whether a step from arrays ``q`` runs on tiles: they are copied in 16-byte pieces, so one
+        installed at an odd offset of its storage takes the two-launch step."""
+        return self._tiles is not None and not any(t.data_ptr() % 16 for t in q)
+
     def _state_key(self):
         return tuple(self.varbs[k].version("cell") for k in ("h", "hu", "hv"))
 
@@ -917,7 +927,7 @@ class ShallowWaterSolver:
         cur, nxt = self._use_dt(), self._slot(1)
         q = _lib.p5([_p(t) for t in qin] + [_p(z)])
         scratch = _p(self._scratch) if self._scratch is not None else None
-        if self._tiles is not None:
+        if self._on_tiles(qin + [z]):
             _lib.call("mb_sw_step_tile", self._dm.struct, self._tiles, q, _lib.p4([_p(t) for t in qout]),
                       float(self.cfl), float(self.grav), int(self.order), _lib.WALLS[self.walls], scratch, _p(cur),
                       _p(nxt), _p(self._slot(2)), self._stream())
@@ -926,6 +936,8 @@ class ShallowWaterSolver:
             _lib.call("mb_sw_step_ex", self._dm.struct, q, _lib.p5([_p(t) for t in qout] + [_p(z)]), float(self.cfl),
                       float(self.grav), int(self.order), _lib.WALLS[self.walls], scratch, _p(self._face_flux()),
                       _p(cur), _p(nxt), self._stream())
+            self._slot(2).fill_(1e6)    # as the step on tiles leaves it
+            self._ff_step = None
         self._spare = [self.varbs[k].swap_cell(t) for k, t in zip(names, qout)]
         self._cur = (self._cur + 1) % 4
         self._dt_key = self._state_key()
@@ -1073,7 +1085,7 @@ class ShallowWaterSolver:
             q = [self.varbs[k].dev("cell") for k in ("h", "hu", "hv", "hc")]
             if self._spare is None:
                 self._spare = [torch.empty_like(t) for t in q]
-            if self._tiles is None:
+            if not self._on_tiles(q + self._spare + [self.Z.dev("cell")]):
                 self._face_flux()
             ptrs = [q, self._spare, [self.Z.dev("cell")]]
         self._use_dt()
@@ -1086,8 +1098,8 @@ class ShallowWaterSolver:
         else:
             for k in ("h", "hu", "hv", "hc"):
                 self.varbs[k]._s.version["cell"] += 1
-            if self._tiles is not None:
-                self._ff_step = (float(self.cfl), float(self.grav))
+            on_tiles = self._on_tiles(self._spare + [self.Z.dev("cell")])     # the last step's arrays
+            self._ff_step = (float(self.cfl), float(self.grav)) if on_tiles else None
         self._dt_key = self._state_key()
         self._dt_host = None
 

@@ -75,3 +75,23 @@ def test_replayed_lengths_continue_single_steps(precision, steps, cuda):
         runs.append([v.cell.copy() for v in vs[:4]] + [np.array(S.stepper())])
     for x, y in zip(*runs):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("name", ["h", "Z"])
+def test_arrays_at_odd_offsets(name, cuda):
+    """A cell array installed 8 bytes into its storage: the steps that read it take the two-launch step."""
+    import torch
+    dom = M.Domain(dim=2, mesh=meshgen.square_triangles(12, seed=3))
+    _, A = _solver(dom, 1, "reflective")
+    _, B = _solver(dom, 1, "reflective")
+    t = A.varbs[name].dev("cell")
+    odd = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:]
+    odd.copy_(t)
+    A.varbs[name].swap_cell(odd)
+    for steps in (1, 2, 8, 8, 8):
+        A.advance(steps)
+        B.advance(steps)
+        assert A.boundary_mass_flux() == B.boundary_mass_flux()
+        assert A.stepper() == B.stepper()
+    for k in A.varbs:
+        assert np.array_equal(A.varbs[k].cell, B.varbs[k].cell)

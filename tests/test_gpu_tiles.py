@@ -99,3 +99,25 @@ def test_uniform_state_stays_exactly_uniform(cuda):
     S.advance(5, graph=False)
     assert S._tiles is not None
     assert np.array_equal(w.cell, np.full(len(el), 0.7))
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_array_at_an_odd_offset(graph, cuda):
+    """A cell array installed 8 bytes into its storage: the steps that read it take the two-launch step."""
+    import torch
+    dom = M.Domain(dim=2, mesh=meshgen.square_triangles(20, seed=4))
+    out = []
+    for odd in (False, True):
+        w, u, v, z = (M.Variable(domain=dom) for _ in range(4))
+        w.cell = np.sin(5 * dom.cells.center[:, 0])
+        u.face, v.face = np.ones(len(u.face)), np.full(len(u.face), 0.5)
+        S = M.AdvectionDiffusionSolver(w, vel=(u, v, z), conf=M.Struct(Dxx=1e-3, Dyy=2e-3, order=2, cfl=0.5,
+                                                                       graph_depth=4))
+        if odd:
+            t = w.dev("cell")
+            x = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)[1:]
+            x.copy_(t)
+            w.swap_cell(x)
+        S.advance(STEPS, graph=graph)
+        out.append(w.cell.copy())
+    assert rel_max(out[1], out[0]) < TOL
