@@ -347,7 +347,7 @@ def cpu_baseline_euler(dom, wl, steps):
 
 
 def run_euler(args, wl):
-    """The 2D Euler Rusanov step (EulerSolver): two launches per step, dt reduced on the device."""
+    """The 2D Euler Rusanov step (EulerSolver), dt reduced on the device."""
     import torch
     world, rank, local = dist_setup(args)
     # warm-up long enough to capture the step graph (GRAPH_DEPTH steps, aligned to 6)
@@ -399,7 +399,8 @@ def run_euler(args, wl):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_source": peak_kind,
                      "traffic": (traffic * wl.cells if traffic else None),
-                     "kernel": "face flux + cell update (2 launches), compulsory traffic %.1f B/cell-update" % ctm},
+                     "kernel": "fused step (%d launches), compulsory traffic %.1f B/cell-update"
+                               % (S.launches_per_step(), ctm)},
         "clocks": ck,
         "gpu_launches": S.launches_per_step() * K,
     }

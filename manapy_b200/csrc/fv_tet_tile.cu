@@ -12,16 +12,18 @@
 // gradient from L2 and recomputes the geometry of every face in its last pass (normals, diamond
 // vectors, centres: 12 vertex rows, 4 centres and about 300 operations per cell).
 //
-// Sums are kept relative to the tile's first cell: G = sum x_j w'_j and S = sum w'_j with x_j its
-// centre offset and w'_j = w_j - w_first, so a vertex or edge is 4 doubles and a list entry 4
-// multiply-adds, and a uniform state has exact zeros.  The cancellation in G - x_i S is that of
-// values a tile apart (some cells), where the earlier sums took absolute values.
+// Sums are kept relative to the tile's first cell and to a value of the tile: G = sum x_j w'_j and
+// S = sum w'_j with x_j the offset of a centre and w'_j = w_j - w_ref, so a vertex or edge is 4 doubles
+// and a list entry 4 multiply-adds, and a uniform state has exact zeros.  w_ref is the tile's value
+// of least magnitude, so |w'_j| <= 2 |w_j| for its cells: the cancellation in G - x_i S is never
+// much above that of the earlier sums, which took the values themselves, wherever a tile holds
+// a steep front, an outlier or a NaN.
 //
 // Large meshes keep the sums in memory (k_tet_sums, k_tet_cell below) and take the same fluxes.
 //
 // Measured (B200, per step in a CUDA graph, three launches -> this): 2,058 tetrahedra 32 -> 15 us,
 // 16,464 34 -> 15.4, 48,000 39 -> 18.2, 93,750 50 -> 33; with the sums in memory 384,000 115 -> 83,
-// 1,572,864 372 -> 259.  k_tet_flux reads 175 B of DRAM per cell and takes 18 us at 384,000 cells
+// 1,572,864 372 -> 259.  k_tet_flux reads 208 B of DRAM per cell and takes 18 us at 384,000 cells
 // where k_f3_phase2 took 45.  The gradient pass is bound by its chain of passes and by reading the
 // cells around a tile (512 threads x 2 blocks; 384 x 2 100-118 us at 384,000 cells, 256 x 3 124).
 #include "fv_tile.cuh"
@@ -106,15 +108,27 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
   tile_after_previous();
   tile_let_next_start();
   const GhostAfter ghost{make_rule(m, bc, w)};
-  const double wref = ld_after(w + c0);
-  for (int k = tid; k < nc; k += kTetThreads) cw[k] = ld_after(w + c0 + k) - wref;
+  for (int k = tid; k < nc; k += kTetThreads) cw[k] = ld_after(w + c0 + k);
 #pragma unroll 4
-  for (int k = tid; k < nout; k += kTetThreads) cw[T + k] = ld_after(w + (k == tid ? first : ld(ext + k))) - wref;
+  for (int k = tid; k < nout; k += kTetThreads) cw[T + k] = ld_after(w + (k == tid ? first : ld(ext + k)));
   __syncthreads();
   if (!tile_bar_wait(bar)) {        // never seen; a bounded wait leaves the output unwritten
     tile_bar_wait(bar);
     return;
   }
+
+  // every warp finds w_ref for itself (no further barrier; NaN never compares less)
+  double wref = INFINITY;
+  for (int k = tid & 31; k < nc; k += 32)
+    if (fabs(cw[k]) < fabs(wref)) wref = cw[k];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double v = __shfl_xor_sync(0xffffffffu, wref, o);
+    if (fabs(v) < fabs(wref) || (fabs(v) == fabs(wref) && v > wref)) wref = v;   // the same one in every lane
+  }
+  if (!isfinite(wref)) wref = 0.;
+  cw[T + t.ext_cap] = wref;         // the lists' padding adds zeros; every warp writes the same
+  __syncwarp();
 
   // four lanes per vertex (its list is about four times an edge's), each a quarter of the list
   for (int k4 = tid; k4 < ((4 * nn + 31) & ~31); k4 += kTetThreads) {
@@ -127,7 +141,7 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
       for (int q = 32 * sub; q < len; q += 128) {
         const int l = row[q];
         const double2 p = xy[l];
-        const double v = cw[l];
+        const double v = cw[l] - wref;
         gx += p.x * v; gy += p.y * v; gz += z[l] * v;
         s += v;
       }
@@ -175,7 +189,7 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
     for (int q = 0; q < len; q += 32) {
       const int l = row[q];
       const double2 p = xy[l];
-      const double v = cw[l];
+      const double v = cw[l] - wref;
       gx += p.x * v; gy += p.y * v; gz += z[l] * v;
       s += v;
     }
@@ -191,7 +205,7 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
     auto entry = [&](int j) { return (int)((words[j >> 1] >> (16 * (j & 1))) & 0xffffu); };
     const double *Q = t.cell_q + i;
     const long long n = m.nbcells;
-    const double wi = cw[k];
+    const double w0 = cw[k], wi = w0 - wref;
     const double2 p = xy[k];
     const double pz = z[k];
     double gx = 0., gy = 0., gz = 0., s = 0.;
@@ -211,7 +225,7 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
       const int o = entry(10 + j);
       double v;
       if (o != kNoCell) {
-        v = cw[o];
+        v = cw[o] - wref;
         const double2 q = xy[o];
         gx += q.x * v; gy += q.y * v; gz += z[o] * v;
         s += v;
@@ -255,7 +269,7 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
       const double ad = fabs(de[j]), room = de[j] > 0. ? up : dn;
       if (ad >= 1e-10 && room * den < num * ad) { num = room; den = ad; }
     }
-    const double ps = num / den, w0 = ld_after(w + i);
+    const double ps = num / den;
     st4_keep(face_values + 4 * (long long)i, w0 + ps * de[0], w0 + ps * de[1], w0 + ps * de[2], w0 + ps * de[3],
              l2_keep());
   }

@@ -17,7 +17,7 @@
 // Measured (B200, per step in a CUDA graph, two-launch step with tuned launch shapes -> this):
 // 2M triangles 187 -> 107 us, 500,000 48.5 -> 33, 180,000 21.4 -> 14.0, 62,658 13.8 -> 7.4, 1,152
 // 11.9 -> 6.2; first order with diffusion 20,000 8.8 -> 4.2; no diffusion 245,000 28 -> 15.
-// It reads 217 B of DRAM per cell-update at 2M cells.  What bounds it is the chain of passes in
+// It moves 225 B of DRAM per cell-update (500,000 cells).  What bounds it is the chain of passes in
 // a block (barriers 30 % of the stalls, bulk copies and smem latency most of the rest; the
 // load/store pipe is 45 % busy, two fifths of that bank conflicts), so three blocks per SM overlap
 // each other's passes.  What was tried on the way, 2M triangles: everything loaded through

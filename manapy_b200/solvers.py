@@ -786,6 +786,7 @@ class ShallowWaterSolver:
             # dt ring: slot _cur holds the dt of the current state when _dt_key matches; the one-launch
             # step mins the next one into the slot after it (1e6 before) and resets the one after that
             self._dt_buf = torch.full((4,), 1e6, dtype=torch.float64, device=dev)
+            self._dt_slots = [self._dt_buf[k:k + 1] for k in range(4)]
             self._cur = 0
             self._dt_key = None
             self._tiles = self._dm.face_tiles(self._stream()) if self.precision == "fp64" else None
@@ -804,8 +805,7 @@ class ShallowWaterSolver:
 
     def _slot(self, k=0):
         """dt ring slot ``k`` after the current one."""
-        at = (self._cur + k) % 4
-        return self._dt_buf[at:at + 1]
+        return self._dt_slots[(self._cur + k) % 4]
 
     def _all_neumann(self):
         return all(var.resolved_bc.all_neumann for var in self.varbs.values())
