@@ -162,8 +162,13 @@ __global__ void __launch_bounds__(kTetThreadsPlan) k_tet_plan(mb_mesh m, mb_tet_
   if (s.bad || nout > t.ext_cap || nn > t.node_cap || ne > t.edge_cap || s.ngrp[ng] > t.ninc_cap ||
       s.egrp[eg] > t.einc_cap)
     return;
-  // coordinates relative to the first cell's centre
-  const D3 org = ld3(m.cell_xy + 4 * (long long)c0);
+  // coordinates relative to the mean of the cells' centres (every warp forms the same)
+  D3 org = {0., 0., 0.};
+  for (int k = tid & 31; k < nc; k += 32) org = org + ld3(m.cell_xy + 4 * (long long)(c0 + k));
+  for (int o = 16; o > 0; o >>= 1)
+    org = org + D3{__shfl_xor_sync(0xffffffffu, org.x, o), __shfl_xor_sync(0xffffffffu, org.y, o),
+                   __shfl_xor_sync(0xffffffffu, org.z, o)};
+  org = (1. / nc) * org;
   auto put_xyz = [&](double *xy, double *z, long long at, int c) {
     const D3 p = ld3(m.cell_xy + 4 * (long long)c);
     reinterpret_cast<double2 *>(xy)[at] = make_double2(p.x - org.x, p.y - org.y);
@@ -243,7 +248,7 @@ __global__ void __launch_bounds__(kTetThreadsPlan) k_tet_plan(mb_mesh m, mb_tet_
 
 // planes of a cell's reconstruction: (de_0, de_1, de_2) = Q J, rows Q_k = (face centre k - centre)^T
 // times the inverse moment matrix (cell_lsq: cofactors, determinant, and D, the sum of the
-// stencil's centre offsets): Q (9 planes), Q D (3)
+// stencil's centre offsets): Q (9 planes), D (3)
 __global__ void __launch_bounds__(kBlock) k_tet_q(mb_mesh m, double *__restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m.nbcells) return;
@@ -251,6 +256,7 @@ __global__ void __launch_bounds__(kBlock) k_tet_q(mb_mesh m, double *__restrict_
   const int4 vt = ld4(m.cell_vtx + 4 * (long long)i);
   const D3 P[4] = {ld3(m.node_coord + 4 * (long long)vt.x), ld3(m.node_coord + 4 * (long long)vt.y),
                    ld3(m.node_coord + 4 * (long long)vt.z), ld3(m.node_coord + 4 * (long long)vt.w)};
+  const uint32_t fl = ld(m.cell_flags + i);
   double a0, a1, a2, a3, a4, a5, dia, pad, Dx, Dy, Dz;
   ld4d(m.cell_lsq + 12 * (long long)i, a0, a1, a2, a3);
   ld4d(m.cell_lsq + 12 * (long long)i + 4, a4, a5, dia, pad);
@@ -258,14 +264,18 @@ __global__ void __launch_bounds__(kBlock) k_tet_q(mb_mesh m, double *__restrict_
   const long long n = m.nbcells;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    const D3 f = (1. / 3) * (P[tet_face(j, 0)] + P[tet_face(j, 1)] + P[tet_face(j, 2)]) - c;
+    int d0, d1, d2;
+    face_desc(fl, j, d0, d1, d2);
+    const D3 f = (1. / 3) * tet_face_sum(P, j, d2) - c;   // rounded as manapy's face centre
     const double qx = (f.x * a0 + f.y * a1 + f.z * a2) / dia, qy = (f.x * a1 + f.y * a3 + f.z * a4) / dia,
                  qz = (f.x * a2 + f.y * a4 + f.z * a5) / dia;
     out[(3 * j) * n + i] = qx;
     out[(3 * j + 1) * n + i] = qy;
     out[(3 * j + 2) * n + i] = qz;
-    out[(9 + j) * n + i] = qx * Dx + qy * Dy + qz * Dz;
   }
+  out[9 * n + i] = Dx;
+  out[10 * n + i] = Dy;
+  out[11 * n + i] = Dz;
 }
 
 __global__ void __launch_bounds__(kBlock) k_tet_tables(mb_mesh m, mb_tet_tables t) {

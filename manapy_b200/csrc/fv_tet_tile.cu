@@ -12,12 +12,13 @@
 // gradient from L2 and recomputes the geometry of every face in its last pass (normals, diamond
 // vectors, centres: 12 vertex rows, 4 centres and about 300 operations per cell).
 //
-// Sums are kept relative to the tile's first cell and to a value of the tile: G = sum x_j w'_j and
-// S = sum w'_j with x_j the offset of a centre and w'_j = w_j - w_ref, so a vertex or edge is 4 doubles
-// and a list entry 4 multiply-adds, and a uniform state has exact zeros.  w_ref is the tile's value
-// of least magnitude, so |w'_j| <= 2 |w_j| for its cells: the cancellation in G - x_i S is never
-// much above that of the earlier sums, which took the values themselves, wherever a tile holds
-// a steep front, an outlier or a NaN.
+// Sums are kept relative to the middle of the tile and of its values: G = sum x_j w'_j and S = sum w'_j
+// with x_j the offset of a centre and w'_j = w_j - w_ref, so a vertex or edge is 4 doubles and a list
+// entry 4 multiply-adds, and a uniform state has exact zeros.  w_ref is the middle of the tile's
+// values if they are of one sign and within a factor of 5, else the least in magnitude, or 0 where
+// they change sign: |w'_j| <= 2 |w_j| for its cells, so the cancellation in G - x_i S is never much
+// above that of the earlier sums, which took the values themselves, wherever a tile holds a steep
+// front, an outlier or a NaN.
 //
 // Large meshes keep the sums in memory (k_tet_sums, k_tet_cell below) and take the same fluxes.
 //
@@ -117,15 +118,22 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
     return;
   }
 
-  // every warp finds w_ref for itself (no further barrier; NaN never compares less)
-  double wref = INFINITY;
-  for (int k = tid & 31; k < nc; k += 32)
-    if (fabs(cw[k]) < fabs(wref)) wref = cw[k];
+  // every warp finds w_ref for itself (no further barrier; NaN compares neither less nor greater)
+  double least = INFINITY, most = -INFINITY;
+  for (int k = tid & 31; k < nc; k += 32) {
+    const double v = cw[k];
+    if (v < least) least = v;
+    if (v > most) most = v;
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
-    const double v = __shfl_xor_sync(0xffffffffu, wref, o);
-    if (fabs(v) < fabs(wref) || (fabs(v) == fabs(wref) && v > wref)) wref = v;   // the same one in every lane
+    const double a = __shfl_xor_sync(0xffffffffu, least, o), c = __shfl_xor_sync(0xffffffffu, most, o);
+    if (a < least) least = a;
+    if (c > most) most = c;
   }
+  double wref = 0.;
+  if (least > 0.) wref = most <= 5. * least ? 0.5 * least + 0.5 * most : least;
+  if (most < 0.) wref = least >= 5. * most ? 0.5 * least + 0.5 * most : most;
   if (!isfinite(wref)) wref = 0.;
   cw[T + t.ext_cap] = wref;         // the lists' padding adds zeros; every warp writes the same
   __syncwarp();
@@ -219,28 +227,27 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
       const double2 a = eG[entry(4 + j)], c = eS[entry(4 + j)];
       gx -= a.x; gy -= a.y; gz -= c.x; s -= c.y;
     }
-    double hi = wi, lo = wi;
+    double hi = w0, lo = w0;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int o = entry(10 + j);
       double v;
       if (o != kNoCell) {
-        v = cw[o] - wref;
+        v = cw[o];
+        const double vr = v - wref;
         const double2 q = xy[o];
-        gx += q.x * v; gy += q.y * v; gz += z[o] * v;
-        s += v;
+        gx += q.x * vr; gy += q.y * vr; gz += z[o] * vr;
+        s += vr;
       } else {
-        v = ghost(-1 - ld(m.cell_nbr + 4 * (long long)i + j)) - wref;
+        v = ghost(-1 - ld(m.cell_nbr + 4 * (long long)i + j));
       }
       hi = pmax(hi, v);
       lo = pmin(lo, v);
     }
-    double jx = gx - p.x * s, jy = gy - p.y * s, jz = gz - pz * s;
     // the stencil's own part, sum (x_j - x_i) w'_j, takes - w'_i D (cell_q's last planes); ghosts are
     // differences as they stand
-    double de[4];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) de[q] = -wi * ld(Q + (9 + q) * n);
+    double jx = (gx - p.x * s) - wi * ld(Q + 9 * n), jy = (gy - p.y * s) - wi * ld(Q + 10 * n),
+           jz = (gz - pz * s) - wi * ld(Q + 11 * n);
     if (entry(14)) {
       const D3 c = ld3(m.cell_xy + 4 * (long long)i);
       const int e = ld(m.ghostnid_ptr + i + 1);
@@ -252,17 +259,18 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
         for (int u = 0; u < 4; ++u) {
           if (f[u] < 0) continue;
           const double *x = m.face_ghostcenter + 3 * (long long)f[u];
-          const double d = (g[u] - wref) - wi;
+          const double d = g[u] - w0;
           jx += (ld(x) - c.x) * d; jy += (ld(x + 1) - c.y) * d; jz += (ld(x + 2) - c.z) * d;
         }
       }
     }
+    double de[4];
 #pragma unroll
     for (int q = 0; q < 3; ++q)
-      de[q] += ld(Q + (3 * q) * n) * jx + ld(Q + (3 * q + 1) * n) * jy + ld(Q + (3 * q + 2) * n) * jz;
+      de[q] = ld(Q + (3 * q) * n) * jx + ld(Q + (3 * q + 1) * n) * jy + ld(Q + (3 * q + 2) * n) * jz;
     de[3] = -((de[0] + de[1]) + de[2]);   // the face centres' mean is the centre
     // Barth limiter (manapy/ast/functions3d.py:364-408), one division as in k_f2_tile
-    const double up = hi - wi, dn = wi - lo;
+    const double up = hi - w0, dn = w0 - lo;
     double num = 1., den = 1.;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
@@ -457,6 +465,7 @@ __global__ void __launch_bounds__(128, MB_TET_CELL_MIN_BLOCKS)
   const double *Q = cell_q + i;
   const long long n = m.nbcells;
   const uint64_t once = l2_stream();
+  sx -= wi * ldd_stream(Q + 9 * n, once); sy -= wi * ldd_stream(Q + 10 * n, once); sz -= wi * ldd_stream(Q + 11 * n, once);
   const int ge = ld(m.ghostnid_ptr + i + 1);
   for (int g = ld(m.ghostnid_ptr + i); g < ge; g += 4) {
     int f[4];
@@ -474,7 +483,7 @@ __global__ void __launch_bounds__(128, MB_TET_CELL_MIN_BLOCKS)
 #pragma unroll
   for (int q = 0; q < 3; ++q)
     de[q] = ldd_stream(Q + (3 * q) * n, once) * sx + ldd_stream(Q + (3 * q + 1) * n, once) * sy +
-            ldd_stream(Q + (3 * q + 2) * n, once) * sz - wi * ldd_stream(Q + (9 + q) * n, once);
+            ldd_stream(Q + (3 * q + 2) * n, once) * sz;
   de[3] = -((de[0] + de[1]) + de[2]);   // the face centres' mean is the centre
   const double up = hi - wi, dn = wi - lo;
   double num = 1., den = 1.;
