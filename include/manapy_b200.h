@@ -368,7 +368,7 @@ typedef struct mb_tet_tiles {
   uint16_t *ninc, *einc;         /* node / edge -> local cells, SELL-32; cells + ext_cap past a list's end */
   uint16_t *cell;                /* [nbcells][16] local nodes (4), local edges (6), local neighbours (4; 0xffff:
                                     boundary face), 1 if the cell has stencil ghosts, 0 */
-  double *cell_q;                /* [12][nbcells] least-squares reconstruction at three faces */
+  double *cell_q;                /* [12][nbcells] least-squares reconstruction at three faces (9), moment offsets D (3) */
   uint16_t *link;                /* [nbcells] bit j left cell of face j, bits 4+2j.. the face in the neighbour */
 } mb_tet_tiles;
 

@@ -510,8 +510,8 @@ class DeviceMesh:
     # Tetrahedra, second order (fv_tet_tile.cu): a B200 runs 148 SMs x 2 blocks of the tiled gradient pass
     # at once; tiles of one or two rounds of blocks, at most 256 cells (shared memory).  A tile has
     # three to five outside cells per cell of its own, so past two rounds the sums in memory are as
-    # fast (16,464 cells: 15.4 against 25.5 us; 93,750: 32.7 / 38.0; 162,000: 50.2 / 50.5; 384,000:
-    # 100 / 83)
+    # fast (16,464 cells: 15.5 against 25.6 us; 48,000: 18.7 / 33.9; 93,750: 34.4 / 38.0; 162,000: 51 / 50;
+    # 384,000: 110 / 81)
     TET_SLOTS = 296
     TET_TILE_CELLS = 256
     TET_TILED = 110_000

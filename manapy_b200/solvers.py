@@ -505,15 +505,18 @@ class AdvectionDiffusionSolver:
     def _call_f32c(self, k, src, st):
         """One step from buffer k into buffer 1 - k."""
         w, lo = self._w32, self._lo32
+        if self._tab32 is not None:
+            _lib.call("mb_advdiff_step_f32c_tab", self._dm.struct, self._tab32, self.var.device_bc.struct, self._params,
+                      _p(w[k]), _p(w[1 - k]), _p(lo[k]), _p(lo[1 - k]), _p(self._sign32), _p(src), _p(self._dt_dev),
+                      _p(self._cs32), _p(self._ns32), st)
+            return
         if self._cs32.numel() < self._dm.cell_scratch_size_f32c():
             # another solver on this mesh opted its struct into the edge sums since the
             # scratch was sized
             self._cs32 = torch.empty(self._dm.cell_scratch_size_f32c(), dtype=torch.float32, device=self._dm.device)
-        name, tab = ("mb_advdiff_step_f32c", ()) if self._tab32 is None else \
-            ("mb_advdiff_step_f32c_tab", (self._tab32,))
-        _lib.call(name, self._dm.struct, *tab, self.var.device_bc.struct, self._params, _p(w[k]), _p(w[1 - k]),
-                  _p(lo[k]), _p(lo[1 - k]), _p(self._sign32), _p(src), _p(self._dt_dev), _p(self._cs32),
-                  _p(self._ns32), st)
+        _lib.call("mb_advdiff_step_f32c", self._dm.struct, self.var.device_bc.struct, self._params, _p(w[k]),
+                  _p(w[1 - k]), _p(lo[k]), _p(lo[1 - k]), _p(self._sign32), _p(src), _p(self._dt_dev),
+                  _p(self._cs32), _p(self._ns32), st)
 
     def _fused_step_f32c(self):
         self._f32_state()
