@@ -707,6 +707,7 @@ class ShallowWaterSolver:
                    ("walls", str, "neumann", 0, "boundary faces of the fused step: neumann (manapy's default "
                                                 "ghosts, the interior state) or reflective (mirrored momentum, "
                                                 "no mass flux; no counterpart in manapy)")]
+    GRAPH_STEPS = 128      # most steps in one graph of advance()
 
     @classmethod
     def process_conf(cls, conf, kwargs):
@@ -1060,21 +1061,23 @@ class ShallowWaterSolver:
             raise NotImplementedError("advance() runs the fused step, which needs Neumann boundaries")
         n = int(nsteps)
         # a length asked for before is replayed from a graph: after 4 k steps every buffer and the dt
-        # ring are where they were
-        steps = n & ~3
-        if steps:
+        # ring are where they were.  Longer runs repeat a graph of GRAPH_STEPS
+        while n >= 4:
+            steps = min(n & ~3, self.GRAPH_STEPS)
             key = (steps,) + self._prime()
             g = self._graphs.get(key)
             if g is not None:
                 g.replay()
                 self._published()
-                n -= steps
-            elif self._graphs.worth(key):
-                def body():
+            else:
+                def body(steps=steps):
                     for _ in range(steps):
                         self._fused_step()
-                self._graphs.capture(key, self._dm.device, body).replay()
-                n -= steps
+                if self._graphs.worth(key):
+                    self._graphs.capture(key, self._dm.device, body).replay()
+                else:
+                    body()
+            n -= steps
         for _ in range(n):
             self._fused_step()
 

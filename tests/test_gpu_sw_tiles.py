@@ -55,7 +55,7 @@ def test_tiled_step_gives_the_two_launch_bits(n, tile, order, walls, monkeypatch
         assert np.array_equal(x.cell, y.cell) and np.isfinite(x.cell).all()
 
 
-@pytest.mark.parametrize("precision,steps", [("fp64", 7), ("fp64", 8), ("fp32c", 10)])
+@pytest.mark.parametrize("precision,steps", [("fp64", 7), ("fp64", 8), ("fp64", 270), ("fp32c", 10)])
 def test_replayed_lengths_continue_single_steps(precision, steps, cuda):
     """advance() of one length again and again (graph replays, odd rests between) against single steps,
     with a field written from the host and dt set by hand in between."""
