@@ -1095,7 +1095,8 @@ class ShallowWaterSolver:
                 self._face_flux()
             ptrs = [q, self._spare, [self.Z.dev("cell")]]
         self._use_dt()
-        return (self._cur, float(self.cfl), float(self.grav)) + tuple(_p(t) for ts in ptrs for t in ts)
+        return (self._cur, float(self.cfl), float(self.grav), int(self.order), self.walls) + \
+            tuple(_p(t) for ts in ptrs for t in ts)
 
     def _published(self):
         """After replayed steps: the state in the buffers it was in is a new one."""
