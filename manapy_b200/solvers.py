@@ -776,7 +776,7 @@ class ShallowWaterSolver:
         self._dm = None
         self._tiles = None
         self._ff = None
-        self._ff_step = None   # (cfl, grav) of the last one-launch step, whose face fluxes are not kept
+        self._ff_step = None   # _options() of the last one-launch step, whose face fluxes are not kept
         self._graphs = _Graphs()
         self._spare = None
         self._scratch = None
@@ -821,6 +821,10 @@ class ShallowWaterSolver:
         """Whether a step from arrays ``q`` runs on tiles: they are copied in 16-byte pieces, so one
         installed at an odd offset of its storage takes the two-launch step."""
         return self._tiles is not None and not any(t.data_ptr() % 16 for t in q)
+
+    def _options(self):
+        """The options a step depends on, as mb_sw_step_split takes them."""
+        return float(self.cfl), float(self.grav), int(self.order), _lib.WALLS[self.walls]
 
     def _state_key(self):
         return tuple(self.varbs[k].version("cell") for k in ("h", "hu", "hv"))
@@ -933,13 +937,11 @@ class ShallowWaterSolver:
         scratch = _p(self._scratch) if self._scratch is not None else None
         if self._on_tiles(qin + [z]):
             _lib.call("mb_sw_step_tile", self._dm.struct, self._tiles, q, _lib.p4([_p(t) for t in qout]),
-                      float(self.cfl), float(self.grav), int(self.order), _lib.WALLS[self.walls], scratch, _p(cur),
-                      _p(nxt), _p(self._slot(2)), self._stream())
-            self._ff_step = (float(self.cfl), float(self.grav))
+                      *self._options(), scratch, _p(cur), _p(nxt), _p(self._slot(2)), self._stream())
+            self._ff_step = self._options()
         else:
-            _lib.call("mb_sw_step_ex", self._dm.struct, q, _lib.p5([_p(t) for t in qout] + [_p(z)]), float(self.cfl),
-                      float(self.grav), int(self.order), _lib.WALLS[self.walls], scratch, _p(self._face_flux()),
-                      _p(cur), _p(nxt), self._stream())
+            _lib.call("mb_sw_step_ex", self._dm.struct, q, _lib.p5([_p(t) for t in qout] + [_p(z)]), *self._options(),
+                      scratch, _p(self._face_flux()), _p(cur), _p(nxt), self._stream())
             self._slot(2).fill_(1e6)    # as the step on tiles leaves it
             self._ff_step = None
         self._spare = [self.varbs[k].swap_cell(t) for k, t in zip(names, qout)]
@@ -1034,13 +1036,15 @@ class ShallowWaterSolver:
             ff = self._ff32.view(-1, 4)[:, 0]
         else:
             if self._ff_step is not None:
-                # the one-launch step keeps no face fluxes: those of its input state (the same bits)
-                z = self.Z.dev("cell")
+                # the one-launch step keeps no face fluxes: those of its input state with its options (the
+                # same bits).  A boundary face has the same bed on both sides, so any will do for the
+                # one that the step saw, which may have been edited since
                 now = [self.varbs[k].dev("cell") for k in ("h", "hu", "hv", "hc")]
-                _lib.call("mb_sw_step_split", dm.struct, _lib.p5([_p(t) for t in self._spare] + [_p(z)]),
-                          _lib.p5([_p(t) for t in now] + [_p(z)]), *self._ff_step, int(self.order),
-                          _lib.WALLS[self.walls], _p(self._scratch) if self._scratch is not None else None,
-                          _p(self._face_flux()), _p(self._slot()), None, 0, 0, self._stream())
+                z = _p(self._spare[0])
+                _lib.call("mb_sw_step_split", dm.struct, _lib.p5([_p(t) for t in self._spare] + [z]),
+                          _lib.p5([_p(t) for t in now] + [z]), *self._ff_step,
+                          _p(self._scratch) if self._scratch is not None else None, _p(self._face_flux()),
+                          _p(self._slot()), None, 0, 0, self._stream())
                 self._ff_step = None
             ff = self._face_flux().view(-1)[:4 * dm.nbfaces].view(-1, 4)[:, 0]
         return float(ff.index_select(0, self._bfaces).double().sum().item())
@@ -1095,8 +1099,7 @@ class ShallowWaterSolver:
                 self._face_flux()
             ptrs = [q, self._spare, [self.Z.dev("cell")]]
         self._use_dt()
-        return (self._cur, float(self.cfl), float(self.grav), int(self.order), self.walls) + \
-            tuple(_p(t) for ts in ptrs for t in ts)
+        return (self._cur,) + self._options() + tuple(_p(t) for ts in ptrs for t in ts)
 
     def _published(self):
         """After replayed steps: the state in the buffers it was in is a new one."""
@@ -1106,7 +1109,7 @@ class ShallowWaterSolver:
             for k in ("h", "hu", "hv", "hc"):
                 self.varbs[k]._s.version["cell"] += 1
             on_tiles = self._on_tiles(self._spare + [self.Z.dev("cell")])     # the last step's arrays
-            self._ff_step = (float(self.cfl), float(self.grav)) if on_tiles else None
+            self._ff_step = self._options() if on_tiles else None
         self._dt_key = self._state_key()
         self._dt_host = None
 
