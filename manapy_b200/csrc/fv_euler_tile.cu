@@ -193,7 +193,7 @@ extern "C" int mb_euler_step_tile(const mb_mesh *m, const mb_face_tiles *t, cons
   a.dt = ring + step % 3; a.dt_next = ring + (step + 1) % 3; a.dt_after = ring + (step + 2) % 3;
   a.time = time;
   a.cfl = cfl; a.gamma = gamma;
-  return tile_launch(k_euler_tile, t->count, kEulerThreads, 8 * EulerTileLayout(*t).total,
+  return tile_launch<k_euler_tile>(t->count, kEulerThreads, 8 * EulerTileLayout(*t).total,
                      reinterpret_cast<cudaStream_t>(stream), *m, *t, a) == cudaSuccess
              ? MB_OK
              : MB_ECUDA;

@@ -222,9 +222,9 @@ extern "C" int mb_sw_step_tile(const mb_mesh *m, const mb_face_tiles *t, const d
     if (rc != MB_OK) return rc;
     for (int k = 0; k < 4; ++k) a.gr[k] = scratch + k * n;
     a.psi = scratch + 4 * n;
-    e = tile_launch(k_sw2_tile<true>, t->count, kSwTileThreads, bytes, st, *m, *t, a);
+    e = tile_launch<k_sw2_tile<true>>(t->count, kSwTileThreads, bytes, st, *m, *t, a);
   } else {
-    e = tile_launch(k_sw2_tile<false>, t->count, kSwTileThreads, bytes, st, *m, *t, a);
+    e = tile_launch<k_sw2_tile<false>>(t->count, kSwTileThreads, bytes, st, *m, *t, a);
   }
   return e == cudaSuccess ? MB_OK : MB_ECUDA;
 }

@@ -525,14 +525,14 @@ int mb_advdiff_step_tet(const mb_mesh *m, const mb_tet_tiles *t, const mb_bc *bc
   const int bytes = 8 * TetLayout(*t).total, fb = ceil_div(m->nbcells, MB_TET_FLUX_BLOCK);
   cudaError_t e;
   if (df) {
-    e = tile_launch(k_tet_grad<true>, t->count, kTetThreads, bytes, st, *m, *t, *bc, w_in, face_values, node_scratch);
+    e = tile_launch<k_tet_grad<true>>(t->count, kTetThreads, bytes, st, *m, *t, *bc, w_in, face_values, node_scratch);
     if (e == cudaSuccess)
-      e = tile_launch(k_tet_flux<true, false>, fb, MB_TET_FLUX_BLOCK, 0, st, *m, t->link, *bc, w_in, w_out, sign_cf, coef,
+      e = tile_launch<k_tet_flux<true, false>>(fb, MB_TET_FLUX_BLOCK, 0, st, *m, t->link, *bc, w_in, w_out, sign_cf, coef,
                       src, dt_dev, face_values, node_scratch, nullptr);
   } else {
-    e = tile_launch(k_tet_grad<false>, t->count, kTetThreads, bytes, st, *m, *t, *bc, w_in, face_values, node_scratch);
+    e = tile_launch<k_tet_grad<false>>(t->count, kTetThreads, bytes, st, *m, *t, *bc, w_in, face_values, node_scratch);
     if (e == cudaSuccess)
-      e = tile_launch(k_tet_flux<false, false>, fb, MB_TET_FLUX_BLOCK, 0, st, *m, t->link, *bc, w_in, w_out, sign_cf, coef,
+      e = tile_launch<k_tet_flux<false, false>>(fb, MB_TET_FLUX_BLOCK, 0, st, *m, t->link, *bc, w_in, w_out, sign_cf, coef,
                       src, dt_dev, face_values, node_scratch, nullptr);
   }
   return e == cudaSuccess ? MB_OK : MB_ECUDA;

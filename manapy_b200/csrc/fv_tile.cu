@@ -301,7 +301,7 @@ template <bool O2, bool DF>
 static int run_tile(const mb_mesh &m, const mb_tiles &t, const mb_bc &bc, const double *w, double *w_out,
                     const double *sign, const double *coef, const double *src, const double *dt, cudaStream_t st) {
   const int bytes = 8 * TileLayout(t, O2, DF).total;
-  return tile_launch(k_f2_tile<O2, DF>, t.count, kTileThreads, bytes, st, m, t, bc, w, w_out, sign, coef, src, dt) ==
+  return tile_launch<k_f2_tile<O2, DF>>(t.count, kTileThreads, bytes, st, m, t, bc, w, w_out, sign, coef, src, dt) ==
                  cudaSuccess
              ? MB_OK
              : MB_ECUDA;

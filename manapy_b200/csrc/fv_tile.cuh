@@ -8,6 +8,8 @@
 // local nodes are the vertices of the T + n1 cells.  All local indices fit 16 bits.
 #pragma once
 
+#include <atomic>
+
 #include "fv_compact.cuh"
 
 namespace mb {
@@ -166,10 +168,32 @@ __device__ __forceinline__ void ghost4(const GhostRule &g, const int32_t *idx, i
   }
 }
 
+// Lets kernel K take all the shared memory that a block of the device may have.  The limit belongs to the
+// kernel, which every solver in the process launches with the bytes of its own tiles, from any
+// thread: it is set to that one value, before the first launch on a device, and never lowered.
+template <auto K>
+inline cudaError_t tile_shared_limit() {
+  static std::atomic<uint64_t> done{0};          // devices, a bit each; beyond 64 it is set every time
+  int dev = 0, most = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  const uint64_t bit = dev < 64 ? 1ull << dev : 0;
+  if (e != cudaSuccess || (done.load(std::memory_order_acquire) & bit)) return e;
+  cudaFuncAttributes fa;
+  if ((e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+  if ((e = cudaFuncGetAttributes(&fa, K)) != cudaSuccess) return e;
+  e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)fa.sharedSizeBytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+  return e;
+}
+
 template <class... P, class... A>
-inline cudaError_t tile_launch(void (*k)(P...), int blocks, int threads, int bytes, cudaStream_t st, A... args) {
-  if (bytes > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+inline cudaError_t tile_launch_ex(const cudaLaunchConfig_t &cfg, void (*k)(P...), A... args) {
+  return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+template <auto K, class... A>
+inline cudaError_t tile_launch(int blocks, int threads, int bytes, cudaStream_t st, A... args) {
+  if (bytes > 48 * 1024) {                       // what every kernel may take
+    const cudaError_t e = tile_shared_limit<K>();
     if (e != cudaSuccess) return e;
   }
   cudaLaunchAttribute at[1];
@@ -182,7 +206,7 @@ inline cudaError_t tile_launch(void (*k)(P...), int blocks, int threads, int byt
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, P(args)...);
+  return tile_launch_ex(cfg, K, args...);
 }
 
 // flags of a cell record of the tiles with faces: bit j left cell of face j, bits 3-8 manapy's order of
