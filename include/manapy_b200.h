@@ -324,6 +324,8 @@ typedef struct mb_tiles {
   int32_t *grp;                  /* [count][grp_cap] offsets of the node lists of 32 nodes each */
   uint16_t *inc;                 /* [count][inc_cap] node -> local cells, SELL-32, a list's first cell past its end */
   double *node_kappa;            /* [nbnodes] sum of the vertex's centre -> vertex weights over its cells */
+  int32_t *late;                 /* NULL, or a word (of the device or of pinned host memory) that becomes 1 when a
+                                    wait for the copies of a tile ran out: its cells were not written */
 } mb_tiles;
 
 /* Sizes of the tiles of a mesh (compact triangle tables): head [count][4]; *status (device,
@@ -370,6 +372,8 @@ typedef struct mb_tet_tiles {
                                     boundary face), 1 if the cell has stencil ghosts, 0 */
   double *cell_q;                /* [12][nbcells] least-squares reconstruction at three faces (9), moment offsets D (3) */
   uint16_t *link;                /* [nbcells] bit j left cell of face j, bits 4+2j.. the face in the neighbour */
+  int32_t *late;                 /* NULL, or a word (of the device or of pinned host memory) that becomes 1 when a
+                                    wait for the copies of a tile ran out: its cells were not written */
 } mb_tet_tiles;
 
 /* Set-up, once per mesh (compact tables, cell_lsq and the edge tables needed): head [count][8], *status as
@@ -515,6 +519,8 @@ typedef struct mb_face_tiles {
                                     bit j left cell of face j, bits 3-8 cell_order, bit 9+j cells.nf is minus the
                                     normal, bit 12 the cell has a boundary face */
   double *cell_ns;               /* [nbcells][2] y_G - y_1, -(x_G - x_1), 1 the cell's second vertex */
+  int32_t *late;                 /* NULL, or a word (of the device or of pinned host memory) that becomes 1 when a
+                                    wait for the copies of a tile ran out: its cells were not written */
 } mb_face_tiles;
 
 /* Sizes: head [count][4]; *status (device, zero before) becomes 1 when the mesh cannot be tiled this
@@ -529,6 +535,10 @@ int mb_face_tile_fill(const mb_mesh *m, const mb_face_tiles *t, void *stream);
 int mb_sw_step_tile(const mb_mesh *m, const mb_face_tiles *t, const double *const q_in[5], double *const q_out[4],
                     double cfl, double grav, int32_t order, int32_t walls, double *scratch, const double *dt_cur,
                     double *dt_next, double *dt_after, void *stream);
+
+/* A wait of the steps on tiles that nothing ends: gives up after `limit` tries (1 .. 4096) and reports
+ * in *late as they do.  To test what reads the word; no counterpart in manapy. */
+int mb_tile_wait_check(int32_t limit, int32_t *late, void *stream);
 
 /* mb_euler_step_2d in one launch on the tiles of m (bit-identical to it): ring, t and time as there. */
 int mb_euler_step_tile(const mb_mesh *m, const mb_face_tiles *t, const double *const q_in[5], double *const q_out[5],

@@ -54,12 +54,13 @@ class MbTiles(ctypes.Structure):
     _fields_ = [("cells", _i32), ("count", _i32), ("face_cap", _i32), ("ext_cap", _i32), ("node_cap", _i32),
                 ("grp_cap", _i32), ("inc_cap", _i32), ("pad_", _i32), ("head", _vp), ("ext", _vp), ("ext_xy", _vp),
                 ("node", _vp), ("count16", _vp), ("node_c", _vp), ("node_mu", _vp), ("cell", _vp), ("cell_q0", _vp),
-                ("cell_q1", _vp), ("grp", _vp), ("inc", _vp), ("node_kappa", _vp)]
+                ("cell_q1", _vp), ("grp", _vp), ("inc", _vp), ("node_kappa", _vp), ("late", _vp)]
 
 
 class MbFaceTiles(ctypes.Structure):
     _fields_ = [("cells", _i32), ("count", _i32), ("out_cap", _i32), ("face_cap", _i32), ("head", _vp), ("out", _vp),
-                ("face", _vp), ("face_n0", _vp), ("face_n1", _vp), ("face_mes", _vp), ("cell", _vp), ("cell_ns", _vp)]
+                ("face", _vp), ("face_n0", _vp), ("face_n1", _vp), ("face_mes", _vp), ("cell", _vp), ("cell_ns", _vp),
+                ("late", _vp)]
 
 
 class MbTetTiles(ctypes.Structure):
@@ -67,7 +68,7 @@ class MbTetTiles(ctypes.Structure):
                 ("ngrp_cap", _i32), ("egrp_cap", _i32), ("ninc_cap", _i32), ("einc_cap", _i32), ("pad_", _i32),
                 ("head", _vp), ("ext", _vp), ("ext_xy", _vp), ("ext_z", _vp), ("own_xy", _vp), ("own_z", _vp),
                 ("node", _vp), ("node_mu", _vp), ("node_kappa", _vp), ("ngrp", _vp), ("egrp", _vp), ("ninc", _vp),
-                ("einc", _vp), ("cell", _vp), ("cell_q", _vp), ("link", _vp)]
+                ("einc", _vp), ("cell", _vp), ("cell_q", _vp), ("link", _vp), ("late", _vp)]
 
 
 class MbTetTables(ctypes.Structure):
@@ -178,6 +179,7 @@ _SIGS = {
     "mb_face_tile_fill": [_M, ctypes.POINTER(MbFaceTiles), _vp],
     "mb_euler_step_tile": [_M, ctypes.POINTER(MbFaceTiles), _P5, _P5, _d, _d, _vp, _i32, _vp, _vp],
     "mb_sw_step_tile": [_M, ctypes.POINTER(MbFaceTiles), _P5, _P4, _d, _d, _i32, _i32, _vp, _vp, _vp, _vp, _vp],
+    "mb_tile_wait_check": [_i32, _vp, _vp],
     "mb_tet_tile_sizes": [_M, _i32, _vp, _vp, _vp],
     "mb_tet_tile_fill": [_M, ctypes.POINTER(MbTetTiles), _vp],
     "mb_tet_tile_bytes": [ctypes.POINTER(MbTetTiles)],

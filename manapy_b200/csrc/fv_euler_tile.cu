@@ -100,10 +100,7 @@ __global__ void __launch_bounds__(kEulerThreads, MB_EULER_TILE_MIN_BLOCKS)
   }
   tile_copies_done();
   __syncthreads();
-  if (!tile_bar_wait(bar)) {        // never seen; a bounded wait leaves the output unwritten
-    tile_bar_wait(bar);
-    return;
-  }
+  if (!tile_arrived(bar, t.late)) return;   // never seen
 
   for (int k = tid; k < nc + n1; k += kEulerThreads) {
     double *s = q + (k < nc ? k : T + k - nc);

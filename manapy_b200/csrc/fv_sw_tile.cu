@@ -102,10 +102,7 @@ __global__ void __launch_bounds__(kSwTileThreads, MB_SW_TILE_MIN_BLOCKS)
   }
   tile_copies_done();
   __syncthreads();
-  if (!tile_bar_wait(bar)) {        // never seen; a bounded wait leaves the output unwritten
-    tile_bar_wait(bar);
-    return;
-  }
+  if (!tile_arrived(bar, t.late)) return;   // never seen
 
   for (int f = tid; f < nf; f += kSwTileThreads) {
     const uint32_t lr = sface[f];

@@ -113,10 +113,7 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
 #pragma unroll 4
   for (int k = tid; k < nout; k += kTetThreads) cw[T + k] = ld_after(w + (k == tid ? first : ld(ext + k)));
   __syncthreads();
-  if (!tile_bar_wait(bar)) {        // never seen; a bounded wait leaves the output unwritten
-    tile_bar_wait(bar);
-    return;
-  }
+  if (!tile_arrived(bar, t.late)) return;   // never seen
 
   // every warp finds w_ref for itself (no further barrier; NaN compares neither less nor greater)
   double least = INFINITY, most = -INFINITY;

@@ -128,10 +128,7 @@ __global__ void __launch_bounds__(kTileThreads, MB_TILE_MIN_BLOCKS)
   for (int k = tid; k < next; k += kTileThreads) tile_copy8(cw + T + k, w + (k == tid ? first : ld(ext + k)));
   tile_copies_done();
   __syncthreads();
-  if (!tile_bar_wait(bar)) {        // never seen; a bounded wait leaves the output unwritten
-    tile_bar_wait(bar);
-    return;
-  }
+  if (!tile_arrived(bar, t.late)) return;   // never seen
 
   for (int k = tid; k < nn; k += kTileThreads) {
     const int gb = sgrp[k >> 5], ge = sgrp[(k >> 5) + 1];

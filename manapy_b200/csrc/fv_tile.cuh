@@ -52,7 +52,8 @@ __device__ __forceinline__ void tile_bulk(void *dst, const void *src, unsigned b
                  : "memory");
 }
 // waits for phase 0 of the barrier; false when the copies have not arrived after `limit` tries
-__device__ __forceinline__ bool tile_bar_wait(uint64_t *bar, int limit = 1 << 22) {
+constexpr int kTileWait = 1 << 22;
+__device__ __forceinline__ bool tile_bar_wait(uint64_t *bar, int limit) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
   for (int k = 0; k < limit; ++k) {
     unsigned ok;
@@ -62,6 +63,17 @@ __device__ __forceinline__ bool tile_bar_wait(uint64_t *bar, int limit = 1 << 22
                  : "memory");
     if (ok) return true;
   }
+  return false;
+}
+// The wait of a step for the copies of its tile.  When it runs out the block reports in *late, waits once
+// more for what is still in flight towards its shared memory, and has to return with its cells
+// unwritten: the state is then not a step's, which the host sees in *late.
+__device__ __forceinline__ bool tile_arrived(uint64_t *bar, int32_t *late, int limit = kTileWait) {
+  if (tile_bar_wait(bar, limit)) return true;
+  // no fence: the host reads the word after the launch has ended (a fence here, though never run, cost
+  // the shallow-water step 1.9 %: 80.6 -> 82.1 us at 1.28M triangles)
+  if (late) asm volatile("st.relaxed.sys.global.s32 [%0], 1;" ::"l"(late) : "memory");
+  tile_bar_wait(bar, limit);
   return false;
 }
 __device__ __forceinline__ void tile_copies_done() { asm volatile("cp.async.wait_all;" ::: "memory"); }

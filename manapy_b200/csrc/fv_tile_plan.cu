@@ -292,6 +292,17 @@ __global__ void __launch_bounds__(kBlock) k_tile_coef(mb_mesh m, mb_bc bc, mb_ad
   out[5 * n + i] = 1 / ld(m.cell_volume + i);
 }
 
+// the wait of a step for copies that were never issued
+__global__ void k_tile_wait_check(int32_t *late, int limit) {
+  __shared__ __align__(16) uint64_t bar;
+  if (threadIdx.x == 0) {
+    tile_bar_init(&bar);
+    tile_bar_expect(&bar, 16);
+  }
+  __syncthreads();
+  tile_arrived(&bar, late, limit);
+}
+
 // ---------------------------------------------------------------- tiles with their faces
 //
 // For the steps that exchange fluxes (shallow water, Euler): a tile's local cells are its own and,
@@ -497,6 +508,13 @@ int mb_face_tile_fill(const mb_mesh *m, const mb_face_tiles *t, void *stream) {
   const int rc = run_face_plan<true>(m, t, nullptr, nullptr, ST(stream));
   if (rc != MB_OK) return rc;
   tile_filled(ST(stream));
+  return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
+}
+
+int mb_tile_wait_check(int32_t limit, int32_t *late, void *stream) {
+  MB_NVTX();
+  if (limit < 1 || limit > 4096 || !late) return MB_EINVAL;
+  k_tile_wait_check<<<1, 32, 0, ST(stream)>>>(late, limit);
   return cudaGetLastError() == cudaSuccess ? MB_OK : MB_ECUDA;
 }
 

@@ -21,6 +21,9 @@ replayed from a CUDA graph.
 """
 from __future__ import annotations
 
+import threading
+import weakref
+
 import numpy as np
 import torch
 
@@ -79,6 +82,46 @@ class _Graphs:
         while len(self.by_key) > self.MOST:
             self.by_key.pop(next(iter(self.by_key)))
         return g
+
+
+class _Watch:
+    """A word in pinned memory that a step on tiles sets when a wait for its copies ran out (its limit is
+    seconds: a fault of the machine, never seen).  The state is not a step's from there on.
+
+    The words come from pages kept for the process (pinning memory takes longer than a small
+    mesh's set-up) and go back with their solver."""
+    PAGE = 1024
+    _lock = threading.Lock()
+    _free = []       # (page, its host view, index)
+
+    def __init__(self):
+        with self._lock:
+            if not self._free:
+                page = torch.zeros(self.PAGE, dtype=torch.int32, pin_memory=True)
+                self._free.extend((page, page.numpy(), k) for k in range(self.PAGE))
+            slot = self._free.pop()
+        weakref.finalize(self, self._give_back, slot)
+        self.page, self.seen, self.at = slot
+        self.seen[self.at] = 0
+
+    @property
+    def word(self):
+        return self.page[self.at:self.at + 1]
+
+    @classmethod
+    def _give_back(cls, slot):
+        cls._free.append(slot)      # may run inside __init__ (a collection): no lock
+
+    def tiles(self, t):
+        """The tables ``t`` of a mesh for a solver that reports here."""
+        own = type(t).from_buffer_copy(t)
+        own.memory = t.memory
+        own.late = self.page.data_ptr() + 4 * self.at
+        return own
+
+    def check(self):
+        if self.seen[self.at]:
+            raise _lib.MbError("a step on tiles waited in vain for its copies: the solver's state is not complete")
 
 
 def check_state(arrays, nonneg=(), names=None):
@@ -188,9 +231,12 @@ class AdvectionDiffusionSolver:
         self._sign32_key = None
         self._src32 = None
         self._src32_key = None
+        self._watch = None
 
     # ------------------------------------------------------------ device helpers
     def _setup(self):
+        if self._watch is not None:
+            self._watch.check()
         if self._dm is None:
             self._dm = self.domain.device_mesh
             if self.order == 2:
@@ -213,6 +259,9 @@ class AdvectionDiffusionSolver:
                         self._tiles = self._dm.tet_tiles(self._stream())
                     if self._tiles is None:
                         self._tables = self._dm.tet_tables(self._stream())
+                if self._tiles is not None:
+                    self._watch = _Watch()
+                    self._tiles = self._watch.tiles(self._tiles)
             if (self._tiles or self._tables) is not None and self.diffusion:
                 self._coef = torch.empty((6 if self.dim == 2 else 8) * self._dm.nbcells, dtype=torch.float64, device=dev)
                 _lib.call("mb_tile_coef" if self.dim == 2 else "mb_tet_coef", self._dm.struct,
@@ -533,6 +582,7 @@ class AdvectionDiffusionSolver:
             check_state([self._w32[self._w32_i]], names=["the FP32 state"])
         else:
             check_state([self.var.dev("cell")], names=["the cell values"])
+        self._setup()
 
     def launches_per_step(self):
         """Kernel launches of one fused step."""
@@ -775,6 +825,7 @@ class ShallowWaterSolver:
         self.signature = self.domain.signature
         self._dm = None
         self._tiles = None
+        self._watch = None
         self._ff = None
         self._ff_step = None   # _options() of the last one-launch step, whose face fluxes are not kept
         self._graphs = _Graphs()
@@ -784,6 +835,8 @@ class ShallowWaterSolver:
         self._fused = False
 
     def _setup(self):
+        if self._watch is not None:
+            self._watch.check()
         if self._dm is None:
             self._dm = self.domain.device_mesh
             dev = self._dm.device
@@ -794,6 +847,9 @@ class ShallowWaterSolver:
             self._cur = 0
             self._dt_key = None
             self._tiles = self._dm.face_tiles(self._stream()) if self.precision == "fp64" else None
+            if self._tiles is not None:
+                self._watch = _Watch()
+                self._tiles = self._watch.tiles(self._tiles)
             if self.order == 2:
                 self._scratch = torch.zeros(5 * self._dm.nbcells, dtype=torch.float64, device=dev)
         return self._dm
@@ -851,6 +907,7 @@ class ShallowWaterSolver:
         slot = self._dt_slot()
         if self._dt_host is None:
             self._dt_host = float(slot.item())
+            self._setup()      # what the steps before it reported, now that they have run
         self.dt = self._dt_host
         return self.dt
 
@@ -935,13 +992,14 @@ class ShallowWaterSolver:
         cur, nxt = self._use_dt(), self._slot(1)
         q = _lib.p5([_p(t) for t in qin] + [_p(z)])
         scratch = _p(self._scratch) if self._scratch is not None else None
+        options = self._options()
         if self._on_tiles(qin + [z]):
-            _lib.call("mb_sw_step_tile", self._dm.struct, self._tiles, q, _lib.p4([_p(t) for t in qout]),
-                      *self._options(), scratch, _p(cur), _p(nxt), _p(self._slot(2)), self._stream())
-            self._ff_step = self._options()
+            _lib.call("mb_sw_step_tile", self._dm.struct, self._tiles, q, _lib.p4([_p(t) for t in qout]), *options,
+                      scratch, _p(cur), _p(nxt), _p(self._slot(2)), self._stream())
+            self._ff_step = options
         else:
-            _lib.call("mb_sw_step_ex", self._dm.struct, q, _lib.p5([_p(t) for t in qout] + [_p(z)]), *self._options(),
-                      scratch, _p(self._face_flux()), _p(cur), _p(nxt), self._stream())
+            _lib.call("mb_sw_step_ex", self._dm.struct, q, _lib.p5([_p(t) for t in qout] + [_p(z)]), *options, scratch,
+                      _p(self._face_flux()), _p(cur), _p(nxt), self._stream())
             self._slot(2).fill_(1e6)    # as the step on tiles leaves it
             self._ff_step = None
         self._spare = [self.varbs[k].swap_cell(t) for k, t in zip(names, qout)]
@@ -1013,6 +1071,7 @@ class ShallowWaterSolver:
         else:
             arrays = [self.varbs[k].dev("cell") for k in ("h", "hu", "hv", "hc")]
         check_state(arrays, nonneg=(0,), names=["h", "hu", "hv", "hc"])
+        self._setup()
 
     def mass(self):
         """FP64 sum of volume x h over the cells (no counterpart in manapy)."""
@@ -1161,10 +1220,13 @@ class EulerSolver:
         self.dt = float(get("dt"))
         self.backend = self.domain.backend
         self._dm = None
+        self._watch = None
         self._graphs = _Graphs()
 
     # ------------------------------------------------------------ state
     def _setup(self):
+        if self._watch is not None:
+            self._watch.check()
         if self._dm is None:
             for k, v in self.varbs.items():
                 if not v.resolved_bc.all_neumann:
@@ -1178,7 +1240,10 @@ class EulerSolver:
             self._ring = torch.full((3,), 1e300, dtype=f64, device=dm.device)
             self._time = torch.zeros(1, dtype=f64, device=dm.device)
             self._tiles = dm.face_tiles(self._stream(), dm.face_tile_cells(dm.nbcells, dm.EULER_TILE_CELLS))
-            if self._tiles is None:
+            if self._tiles is not None:
+                self._watch = _Watch()
+                self._tiles = self._watch.tiles(self._tiles)
+            else:
                 # the two-launch step: face fluxes, and its static tables (face records, left-cell bits)
                 self._ff = torch.empty(4 * dm.nbfaces, dtype=f64, device=dm.device)
                 self._frec = torch.empty(4 * dm.nbfaces, dtype=f64, device=dm.device)
@@ -1220,6 +1285,7 @@ class EulerSolver:
         self._sync()
         if self._dt_host is None:
             self._dt_host = float(self._slot().item())
+            self._setup()      # what the steps before it reported, now that they have run
         self.dt = self._dt_host
         return self.dt
 
@@ -1307,6 +1373,7 @@ class EulerSolver:
         """Raise if a variable holds NaN or infinity, or rho or P is negative."""
         self._sync()
         check_state([self.varbs[k].dev("cell") for k in self._NAMES], nonneg=(0, 1), names=list(self._NAMES))
+        self._setup()
 
     def launches_per_step(self):
         return 2 if self._dm is None or self._tiles is None else 1
