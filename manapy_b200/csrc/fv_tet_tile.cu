@@ -266,15 +266,7 @@ __global__ void __launch_bounds__(kTetThreads, MB_TET_MIN_BLOCKS)
     for (int q = 0; q < 3; ++q)
       de[q] = ld(Q + (3 * q) * n) * jx + ld(Q + (3 * q + 1) * n) * jy + ld(Q + (3 * q + 2) * n) * jz;
     de[3] = -((de[0] + de[1]) + de[2]);   // the face centres' mean is the centre
-    // Barth limiter (manapy/ast/functions3d.py:364-408), one division as in k_f2_tile
-    const double up = hi - w0, dn = w0 - lo;
-    double num = 1., den = 1.;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const double ad = fabs(de[j]), room = de[j] > 0. ? up : dn;
-      if (ad >= 1e-10 && room * den < num * ad) { num = room; den = ad; }
-    }
-    const double ps = num / den;
+    const double ps = tile_barth(de, hi - w0, w0 - lo, 1e-10);
     st4_keep(face_values + 4 * (long long)i, w0 + ps * de[0], w0 + ps * de[1], w0 + ps * de[2], w0 + ps * de[3],
              l2_keep());
   }
@@ -482,14 +474,7 @@ __global__ void __launch_bounds__(128, MB_TET_CELL_MIN_BLOCKS)
     de[q] = ldd_stream(Q + (3 * q) * n, once) * sx + ldd_stream(Q + (3 * q + 1) * n, once) * sy +
             ldd_stream(Q + (3 * q + 2) * n, once) * sz;
   de[3] = -((de[0] + de[1]) + de[2]);   // the face centres' mean is the centre
-  const double up = hi - wi, dn = wi - lo;
-  double num = 1., den = 1.;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const double ad = fabs(de[j]), room = de[j] > 0. ? up : dn;
-    if (ad >= 1e-10 && room * den < num * ad) { num = room; den = ad; }
-  }
-  const double ps = num / den;
+  const double ps = tile_barth(de, hi - wi, wi - lo, 1e-10);
   st4_keep(face_values + 4 * (long long)i, wi + ps * de[0], wi + ps * de[1], wi + ps * de[2], wi + ps * de[3],
            l2_keep());
 }

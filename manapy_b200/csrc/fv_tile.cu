@@ -227,16 +227,7 @@ __global__ void __launch_bounds__(kTileThreads, MB_TILE_MIN_BLOCKS)
       de[0] = Q0.x * jx + Q0.y * jy;
       de[1] = Q1.x * jx + Q1.y * jy;
       de[2] = -(de[0] + de[1]);
-      // Barth limiter (manapy/ast/functions2d.py:280-325): the smallest of 1 and the three
-      // (bound - w) / delta, found by cross-multiplication so that one division is left
-      const double up = hi - wi, dn = wi - lo;
-      double num = 1., den = 1.;
-#pragma unroll
-      for (int j = 0; j < 3; ++j) {
-        const double ad = fabs(de[j]), room = de[j] > 0. ? up : dn;
-        if (ad >= 1e-8 && room * den < num * ad) { num = room; den = ad; }
-      }
-      const double ps = num / den;
+      const double ps = tile_barth(de, hi - wi, wi - lo, 1e-8);
       q0[li] = make_double2(wi + ps * de[0], wi + ps * de[1]);
       q1[li].x = wi + ps * de[2];
     }

@@ -198,6 +198,35 @@ inline cudaError_t tile_shared_limit() {
   return e;
 }
 
+// Barth limiter of a cell (manapy/ast/functions2d.py:280-325, functions3d.py:364-408): the smallest of 1 and of
+// room / |de_j| over the faces whose offset de_j is `least` or more, room = up where the offset is
+// positive, else dn.  Found by multiplying across, so that one division is left.  Those products could
+// overflow where an offset is above 2^510 (3e153): there every quotient is formed.  The offsets sum
+// to zero, so the others bound the last one.  (2M triangles 109.9 us a step without the branch, 109.7
+// with it; 110.5-110.7 with the branch around both ways of finding it.)
+template <int N>
+__device__ __forceinline__ double tile_barth(const double (&de)[N], double up, double dn, double least) {
+  double num = 1., den = 1.;
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    const double ad = fabs(de[j]), room = de[j] > 0. ? up : dn;
+    if (ad >= least && room * den < num * ad) { num = room; den = ad; }
+  }
+  double most = fabs(de[0]);
+#pragma unroll
+  for (int j = 1; j + 1 < N; ++j) most += fabs(de[j]);
+  double ps = num / den;
+  if (__double2hiint(most) >= 0x5fd00000) {
+    ps = 1.;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      const double ad = fabs(de[j]), r = (de[j] > 0. ? up : dn) / ad;
+      if (ad >= least && r < ps) ps = r;
+    }
+  }
+  return ps;
+}
+
 template <class... P, class... A>
 inline cudaError_t tile_launch_ex(const cudaLaunchConfig_t &cfg, void (*k)(P...), A... args) {
   return cudaLaunchKernelEx(&cfg, k, P(args)...);
