@@ -818,7 +818,10 @@ __global__ void __launch_bounds__(kBlock) k_sign_f32c(mb_mesh m, const double *_
 // 2M triangles 180 -> 140, 500,000 43.8 -> 35.5 (first order 23.1 -> 17.4); 1.57M tetrahedra
 // 409 -> 353, 384,000 128 -> 116 (first order 41.7 -> 27.6).
 
-__device__ __forceinline__ unsigned f32c_link(const mb_mesh &m, int i) {
+// bit j left cell of face j, bits 4 + 2 j the face in the neighbour, and (with diffusion) bit 12 + j the face
+// carries a diffusive gradient: a coefficient of zero does not tell, n.D n is zero at 45 degrees
+// where D_xx = -D_yy while the tangential term is not
+__device__ __forceinline__ unsigned f32c_link(const mb_mesh &m, const mb_bc &bc, bool diffusion, int i) {
   const int4 nb = ld4(m.cell_nbr + 4 * (long long)i);
   const uint32_t fl = ld(m.cell_flags + i);
   unsigned link = 0;
@@ -829,6 +832,7 @@ __device__ __forceinline__ unsigned f32c_link(const mb_mesh &m, int i) {
       const int4 back = ld4(m.cell_nbr + 4 * (long long)o);
       link |= (unsigned)(back.x == i ? 0 : (back.y == i ? 1 : (back.z == i ? 2 : 3))) << (4 + 2 * j);
     }
+    if (diffusion && (o >= 0 || ld(bc.face_grad_on + (-1 - o)))) link |= 1u << (12 + j);
   }
   return link;
 }
@@ -843,7 +847,7 @@ __global__ void __launch_bounds__(kBlock) k_f2c_tables(mb_mesh m, mb_bc bc, mb_a
   const uint32_t fl = ld(m.cell_flags + i);
   const double2 P0 = ldd2(m.node_coord + 2 * (long long)vt.x), P1 = ldd2(m.node_coord + 2 * (long long)vt.y),
                 P2 = ldd2(m.node_coord + 2 * (long long)vt.z);
-  t.link[i] = (uint16_t)f32c_link(m, i);
+  t.link[i] = (uint16_t)f32c_link(m, bc, p.diffusion != 0, i);
   for (int j = 1; j < 3; ++j)     // the link's search for a face takes the neighbours as distinct
     for (int q = 0; q < j; ++q)
       if (comp(nb, j) >= 0 && comp(nb, j) == comp(nb, q)) atomicMax(t.status, 1);
@@ -1037,7 +1041,7 @@ __global__ void __launch_bounds__(128, 8)
     for (int j = 0; j < NF; ++j) {
       if (DIM == 2) {
         const float A = ldf_stream(t.coef + j * n + i, pst), O = ldf_stream(t.coef + (3 + j) * n + i, pst);
-        if (O != 0.f) q[j] = A * (v[j] - v[(j + 1) % 3]) + O * dv[j];   // 0: a face without a gradient
+        if (link >> (12 + j) & 1u) q[j] = A * (v[j] - v[(j + 1) % 3]) + O * dv[j];
       } else {
         const float ca = ldf_stream(t.coef + (3 * j) * n + i, pst), cb = ldf_stream(t.coef + (3 * j + 1) * n + i, pst),
                     cr = ldf_stream(t.coef + (3 * j + 2) * n + i, pst);
@@ -1046,7 +1050,7 @@ __global__ void __launch_bounds__(128, 8)
         const bool swp = (fl >> (6 * j + 4)) & 1u;
         const float VA = pick4v(v[0], v[1], v[2], v[3], d0), VB = pick4v(v[0], v[1], v[2], v[3], swp ? d2 : d1),
                     VC = pick4v(v[0], v[1], v[2], v[3], swp ? d1 : d2);
-        if (cr != 0.f) q[j] = ca * (VA - VC) + cb * (VB - VC) + cr * dv[j];
+        if (link >> (12 + j) & 1u) q[j] = ca * (VA - VC) + cb * (VB - VC) + cr * dv[j];
       }
     }
   }
@@ -1084,7 +1088,7 @@ __global__ void __launch_bounds__(kBlock) k_f3c_tables(mb_mesh m, mb_bc bc, mb_a
   const int4 vt = ld4(m.cell_vtx + 4 * (long long)i), nb = ld4(m.cell_nbr + 4 * (long long)i);
   const uint32_t fl = ld(m.cell_flags + i);
   const D3 ci = ld3(m.cell_xy + 4 * (long long)i);
-  t.link[i] = (uint16_t)f32c_link(m, i);
+  t.link[i] = (uint16_t)f32c_link(m, bc, p.diffusion != 0, i);
   for (int j = 1; j < 4; ++j)
     for (int q = 0; q < j; ++q)
       if (comp(nb, j) >= 0 && comp(nb, j) == comp(nb, q)) atomicMax(t.status, 1);
