@@ -44,7 +44,7 @@ class _Graphs:
 
     def __init__(self):
         self.by_key = {}
-        self.seen = []
+        self.seen = {}       # keys asked for once, the last MOST
 
     def clear(self):
         self.by_key.clear()
@@ -58,11 +58,21 @@ class _Graphs:
 
     def worth(self, key):
         """Whether a run of this key was asked for before: a capture costs about what launching its
-        steps one by one does, so a length seen once is not captured."""
-        if key in self.seen:
+        steps one by one does, so a length seen once is not captured, nor one that comes back after
+        more others than graphs are kept: its graph would be gone before its next use."""
+        if self.seen.pop(key, False):
             return True
-        self.seen = (self.seen + [key])[-2 * self.MOST:]
+        self.seen[key] = True
+        self._trim(self.seen)
         return False
+
+    def keep(self, key, g):
+        self.by_key[key] = g
+        self._trim(self.by_key)
+
+    def _trim(self, d):
+        while len(d) > self.MOST:
+            d.pop(next(iter(d)))
 
     def capture(self, key, device, body):
         s = torch.cuda.Stream(device=device)
@@ -78,9 +88,7 @@ class _Graphs:
             finally:
                 g.capture_end()
         cur.wait_stream(s)
-        self.by_key[key] = g
-        while len(self.by_key) > self.MOST:
-            self.by_key.pop(next(iter(self.by_key)))
+        self.keep(key, g)
         return g
 
 
