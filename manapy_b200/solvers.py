@@ -405,7 +405,9 @@ class AdvectionDiffusionSolver:
         if getattr(self, "_cs", None) is None or self._cs.numel() < need:
             # 4 nbcells (2D: records; 3D on tiles: face values) or 8 nbcells (3D: records, rows), plus the vertex and edge
             # records when the 3D step uses the edge sums (grown if another solver on this mesh
-            # opted the struct into them since)
+            # opted the struct into them since).  Graphs hold the addresses of the scratch they were
+            # captured with, which goes back to the allocator here
+            self._graphs.clear()
             self._cs = torch.empty(need, dtype=torch.float64, device=dm.device)
             self._ns = torch.empty(dm.nbnodes, dtype=torch.float64, device=dm.device)
         return self._cs, self._ns
@@ -569,7 +571,8 @@ class AdvectionDiffusionSolver:
             return
         if self._cs32.numel() < self._dm.cell_scratch_size_f32c():
             # another solver on this mesh opted its struct into the edge sums since the
-            # scratch was sized
+            # scratch was sized (graphs hold the old one's address)
+            self._graphs.clear()
             self._cs32 = torch.empty(self._dm.cell_scratch_size_f32c(), dtype=torch.float32, device=self._dm.device)
         _lib.call("mb_advdiff_step_f32c", self._dm.struct, self.var.device_bc.struct, self._params, _p(w[k]),
                   _p(w[1 - k]), _p(lo[k]), _p(lo[1 - k]), _p(self._sign32), _p(src), _p(self._dt_dev),
