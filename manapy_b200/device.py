@@ -418,9 +418,7 @@ class DeviceMesh:
         cells = self.tile_cells(self.nbcells) if cells is None else int(cells)
         if getattr(self, "_tiles", None) is None:
             self._tiles = {}
-        if cells not in self._tiles:
-            self._tiles[cells] = self._build_tiles(cells, stream)
-        return self._tiles[cells]
+        return self._kept(self._tiles, cells, self._build_tiles, cells, stream)
 
     def _build_tiles(self, cells, stream):
         need = ("cell_vtx", "cell_xy", "n2c_ptr", "n2c_alpha", "n2g_ptr", "n2g_alpha", "lsq_sell_idx", "ghostnid_ptr",
@@ -462,9 +460,7 @@ class DeviceMesh:
         cells = self.face_tile_cells(self.nbcells) if cells is None else int(cells)
         if getattr(self, "_face_tiles", None) is None:
             self._face_tiles = {}
-        if cells not in self._face_tiles:
-            self._face_tiles[cells] = self._build_face_tiles(cells, stream)
-        return self._face_tiles[cells]
+        return self._kept(self._face_tiles, cells, self._build_face_tiles, cells, stream)
 
     # a B200 runs 148 SMs x 5 blocks of that kernel at once; with larger tiles fewer blocks fit an
     # SM's shared memory (1.28M cells: 256 cells 80 us, 288 93).  One round of blocks where the mesh
@@ -528,9 +524,7 @@ class DeviceMesh:
         cells = self.tet_tile_cells(self.nbcells) if cells is None else int(cells)
         if getattr(self, "_tet_tiles", None) is None:
             self._tet_tiles = {}
-        if cells not in self._tet_tiles:
-            self._tet_tiles[cells] = self._build_tet_tiles(cells, stream)
-        return self._tet_tiles[cells]
+        return self._kept(self._tet_tiles, cells, self._build_tet_tiles, cells, stream)
 
     def _build_tet_tiles(self, cells, stream):
         need = ("cell_vtx", "cell_xy", "n2c_ptr", "n2c_alpha", "n2g_ptr", "ghostnid_ptr", "face_ghostcenter", "cell_lsq",
@@ -570,22 +564,33 @@ class DeviceMesh:
         the device on first use (with ``cell_lsq`` and the edge tables in the struct); None where it
         does not apply."""
         if getattr(self, "_tet_tables", None) is None:
-            need = ("cell_lsq", "cell_edges", "edge_sell_idx", "n2c_sum_idx", "n2c_ptr", "n2c_alpha", "n2g_ptr",
-                    "ghostnid_ptr", "face_ghostcenter")
-            got = False
-            if self.dim == 3 and self.device is not None and self.stencil == "shared" and \
-                    all(n in self.t for n in need):
-                nc, nn = self.nbcells, self.nbnodes
-                status = torch.zeros(1, dtype=torch.int32, device=self.device)
-                t = _lib.MbTetTables()
-                buf = self._carve(t, {"cell_q": 96 * nc, "link": 2 * nc, "node_mu": 32 * nn})
-                t.status = status.data_ptr()
-                st = stream if stream is not None else torch.cuda.current_stream(self.device).cuda_stream
-                _lib.call("mb_tet_tables_fill", self.struct, t, st)
-                if not int(status.item()):
-                    got = self._filled(t, status, buf, st)
-            self._tet_tables = got
-        return self._tet_tables or None
+            self._tet_tables = {}
+        return self._kept(self._tet_tables, None, self._build_tet_tables, stream)
+
+    def _build_tet_tables(self, stream):
+        need = ("cell_lsq", "cell_edges", "edge_sell_idx", "n2c_sum_idx", "n2c_ptr", "n2c_alpha", "n2g_ptr",
+                "ghostnid_ptr", "face_ghostcenter")
+        if self.dim != 3 or self.device is None or self.stencil != "shared" or any(n not in self.t for n in need):
+            return None
+        nc, nn = self.nbcells, self.nbnodes
+        status = torch.zeros(1, dtype=torch.int32, device=self.device)
+        t = _lib.MbTetTables()
+        buf = self._carve(t, {"cell_q": 96 * nc, "link": 2 * nc, "node_mu": 32 * nn})
+        t.status = status.data_ptr()
+        st = stream if stream is not None else torch.cuda.current_stream(self.device).cuda_stream
+        _lib.call("mb_tet_tables_fill", self.struct, t, st)
+        return None if int(status.item()) else self._filled(t, status, buf, st)
+
+    @staticmethod
+    def _kept(tables, key, build, *args):
+        """``tables[key]``, built on first use; None, and not kept, where the device has no memory left for
+        them: the step that needs no tables then runs, as it does on every mesh that fits."""
+        if key not in tables:
+            try:
+                tables[key] = build(*args)
+            except torch.OutOfMemoryError:
+                return None
+        return tables[key]
 
     def _filled(self, t, head, buf, st):
         """``t`` with the memory that its pointers name, once its tables are there: solvers on other

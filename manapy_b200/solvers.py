@@ -267,13 +267,18 @@ class AdvectionDiffusionSolver:
                         self._tiles = self._dm.tet_tiles(self._stream())
                     if self._tiles is None:
                         self._tables = self._dm.tet_tables(self._stream())
-                if self._tiles is not None:
-                    self._watch = _Watch()
-                    self._tiles = self._watch.tiles(self._tiles)
             if (self._tiles or self._tables) is not None and self.diffusion:
-                self._coef = torch.empty((6 if self.dim == 2 else 8) * self._dm.nbcells, dtype=torch.float64, device=dev)
-                _lib.call("mb_tile_coef" if self.dim == 2 else "mb_tet_coef", self._dm.struct,
-                          self.var.device_bc.struct, self._params, _p(self._coef), self._stream())
+                try:
+                    self._coef = torch.empty((6 if self.dim == 2 else 8) * self._dm.nbcells, dtype=torch.float64,
+                                             device=dev)
+                except torch.OutOfMemoryError:
+                    self._tiles = self._tables = None
+                else:
+                    _lib.call("mb_tile_coef" if self.dim == 2 else "mb_tet_coef", self._dm.struct,
+                              self.var.device_bc.struct, self._params, _p(self._coef), self._stream())
+            if self._tiles is not None:
+                self._watch = _Watch()
+                self._tiles = self._watch.tiles(self._tiles)
         return self._dm
 
     def _stream(self):
@@ -508,7 +513,8 @@ class AdvectionDiffusionSolver:
 
     def _f32_tables(self):
         """The FP32 step's coefficients (``_lib.MbF32cTables``), formed once; None where the step forms
-        them itself (tetrahedra at second order without the edge sums, or a missing table)."""
+        them itself (tetrahedra at second order without the edge sums, a missing table, or no memory
+        left for them)."""
         dm = self._dm
         self._tab32 = None
         need = ("cell_vtx", "ghostnid_ptr", "face_ghostcenter", "lsq_sell_idx", "n2c_sell_alpha_f32")
@@ -522,7 +528,10 @@ class AdvectionDiffusionSolver:
         if dm.dim == 2 and self.order == 2:
             sizes["geom"] = f * 9 * n
         t = _lib.MbF32cTables()
-        buf = dm._carve(t, sizes)
+        try:
+            buf = dm._carve(t, sizes)
+        except torch.OutOfMemoryError:
+            return
         status = torch.zeros(1, dtype=torch.int32, device=dm.device)
         t.status = _p(status)
         _lib.call("mb_f32c_tables_fill", dm.struct, self.var.device_bc.struct, self._params, t, self._stream())
