@@ -38,6 +38,12 @@ def _p(t):
     return t.data_ptr() if t is not None else None
 
 
+def _capturing():
+    """Whether the program captures a graph of its own on the current stream: steps are launched into it
+    then, since neither a capture nor a replay can be part of one."""
+    return torch.cuda.is_current_stream_capturing()
+
+
 class _Graphs:
     """Captured CUDA graphs of a solver by key, the last few used."""
     MOST = 6
@@ -639,8 +645,7 @@ class AdvectionDiffusionSolver:
         if self._spare is None:
             self._spare = torch.empty_like(var.dev("cell"))
         total = n
-        if graph:
-            a = self._graph_bufs[0] if self._graph_bufs else var.dev("cell")
+        if graph and not _capturing():
             if n and self._graph_bufs and var.dev("cell") is self._graph_bufs[1]:
                 self._fused_step()      # after an odd number of steps: one brings the state back to a
                 n -= 1
@@ -671,7 +676,7 @@ class AdvectionDiffusionSolver:
         return n * self._dt_host
 
     def _advance_f32c(self, n, graph):
-        if graph and n:
+        if graph and n and not _capturing():
             depth = self._depth()
             self._f32_state()
             if self._w32_i != 0:  # the captured steps start from buffer 0
@@ -1145,7 +1150,7 @@ class ShallowWaterSolver:
         n = int(nsteps)
         # a length asked for before is replayed from a graph: after 4 k steps every buffer and the dt
         # ring are where they were.  Longer runs repeat a graph of GRAPH_STEPS
-        while n >= 4:
+        while n >= 4 and not _capturing():
             steps = min(n & ~3, self.GRAPH_STEPS)
             key = (steps,) + self._prime()
             g = self._graphs.get(key)
