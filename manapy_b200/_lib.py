@@ -220,6 +220,10 @@ _SIGS = {
     "mb_advdiff_batch_step": [_vp, _vp, _i32, _vp, _i32, _i32, _i32, _vp, _vp],
     "mb_sw_batch_step": [_vp, _vp, _i32, _vp, _i32, _vp, _vp],
     "mb_check_state": [_vp, _vp, ctypes.c_int64, _i32, _vp, _vp],
+    "mb_graph_begin": [ctypes.POINTER(_vp)],
+    "mb_graph_end": [_vp, ctypes.POINTER(_vp)],
+    "mb_graph_launch": [_vp, _vp],
+    "mb_graph_free": [_vp],
     "mb_halo_pack": [_vp, _i32, _vp, ctypes.c_int64, _vp, _vp],
     "mb_halo_unpack": [_vp, _i32, _vp, ctypes.c_int64, _vp, _vp],
     "mb_build_info": [],

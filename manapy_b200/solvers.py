@@ -21,6 +21,7 @@ replayed from a CUDA graph.
 """
 from __future__ import annotations
 
+import ctypes
 import threading
 import weakref
 
@@ -42,6 +43,19 @@ def _capturing():
     """Whether the program captures a graph of its own on the current stream: steps are launched into it
     then, since neither a capture nor a replay can be part of one."""
     return torch.cuda.is_current_stream_capturing()
+
+
+class _Graph:
+    """A captured CUDA graph."""
+
+    def __init__(self, handle, device):
+        self.handle, self.device, self.free = handle, device, _lib.lib().mb_graph_free
+
+    def replay(self):
+        _lib.call("mb_graph_launch", self.handle, torch.cuda.current_stream(self.device).cuda_stream)
+
+    def __del__(self):
+        self.free(self.handle)      # a launch still running ends first
 
 
 class _Graphs:
@@ -81,19 +95,21 @@ class _Graphs:
             d.pop(next(iter(d)))
 
     def capture(self, key, device, body):
-        s = torch.cuda.Stream(device=device)
-        cur = torch.cuda.current_stream(device)
-        s.wait_stream(cur)
-        g = torch.cuda.CUDAGraph()
-        with torch.cuda.stream(s):
-            # relaxed: what Python frees meanwhile (another solver's graph in a garbage collection, a
-            # thread's pinned buffer) must not invalidate the capture; the body only launches
-            g.capture_begin(capture_error_mode="relaxed")
+        """The launches of ``body`` as a graph, kept under ``key``.  Not through torch's graphs: theirs
+        register with the process's random number generator, which only one thread may do at a time
+        (a second one's capture raised, and its destructor ended the process), and capture on
+        streams of a pool that other threads use."""
+        stream, handle, done = ctypes.c_void_p(), ctypes.c_void_p(), False
+        with torch.cuda.device(device):
+            _lib.call("mb_graph_begin", ctypes.byref(stream))
             try:
-                body()
+                with torch.cuda.stream(torch.cuda.ExternalStream(stream.value, device=device)):
+                    body()
+                done = True
             finally:
-                g.capture_end()
-        cur.wait_stream(s)
+                rc = _lib.lib().mb_graph_end(stream, ctypes.byref(handle) if done else None)
+        _lib.check(rc, "mb_graph_end")
+        g = _Graph(handle, device)
         self.keep(key, g)
         return g
 
