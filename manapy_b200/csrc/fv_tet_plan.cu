@@ -252,11 +252,9 @@ __global__ void __launch_bounds__(kTetThreadsPlan) k_tet_plan(mb_mesh m, mb_tet_
 __global__ void __launch_bounds__(kBlock) k_tet_q(mb_mesh m, double *__restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m.nbcells) return;
-  const D3 c = ld3(m.cell_xy + 4 * (long long)i);
   const int4 vt = ld4(m.cell_vtx + 4 * (long long)i);
   const D3 P[4] = {ld3(m.node_coord + 4 * (long long)vt.x), ld3(m.node_coord + 4 * (long long)vt.y),
                    ld3(m.node_coord + 4 * (long long)vt.z), ld3(m.node_coord + 4 * (long long)vt.w)};
-  const uint32_t fl = ld(m.cell_flags + i);
   double a0, a1, a2, a3, a4, a5, dia, pad, Dx, Dy, Dz;
   ld4d(m.cell_lsq + 12 * (long long)i, a0, a1, a2, a3);
   ld4d(m.cell_lsq + 12 * (long long)i + 4, a4, a5, dia, pad);
@@ -264,9 +262,10 @@ __global__ void __launch_bounds__(kBlock) k_tet_q(mb_mesh m, double *__restrict_
   const long long n = m.nbcells;
 #pragma unroll
   for (int j = 0; j < 3; ++j) {
-    int d0, d1, d2;
-    face_desc(fl, j, d0, d1, d2);
-    const D3 f = (1. / 3) * tet_face_sum(P, j, d2) - c;   // rounded as manapy's face centre
+    // face centre - centre: a twelfth of the differences to the opposite vertex o, which round to the
+    // size of the cell, not to that of its coordinates as a difference of two centres does
+    const int o = j == 0 ? 3 : (j == 1 ? 1 : 2);
+    const D3 f = (1. / 12) * (((P[0] - P[o]) + (P[1] - P[o])) + ((P[2] - P[o]) + (P[3] - P[o])));
     const double qx = (f.x * a0 + f.y * a1 + f.z * a2) / dia, qy = (f.x * a1 + f.y * a3 + f.z * a4) / dia,
                  qz = (f.x * a2 + f.y * a4 + f.z * a5) / dia;
     out[(3 * j) * n + i] = qx;

@@ -162,12 +162,13 @@ __global__ void __launch_bounds__(kTileThreads) k_tile_plan(mb_mesh m, mb_tiles 
     const long long at = (long long)blockIdx.x * (T + t.face_cap) + li;
     reinterpret_cast<uint4 *>(t.cell)[at] = u;
     // (de_0, de_1) = Q J: reconstruction offsets at the first two faces from the right-hand side
-    const double2 c = ldd2(m.cell_xy + 2 * (long long)i);
+    // (a face's centre minus the cell's: a sixth of the differences to the opposite vertex, which round to
+    // the size of the cell, not to that of its coordinates)
     const double2 X0 = ldd2(m.node_coord + 2 * (long long)vt.x), X1 = ldd2(m.node_coord + 2 * (long long)vt.y),
                   X2 = ldd2(m.node_coord + 2 * (long long)vt.z);
     const double ia = minv[4 * (long long)i], ib = minv[4 * (long long)i + 1], ic = minv[4 * (long long)i + 2];
-    const double ax = 0.5 * (X0.x + X1.x) - c.x, ay = 0.5 * (X0.y + X1.y) - c.y;
-    const double bx = 0.5 * (X1.x + X2.x) - c.x, by = 0.5 * (X1.y + X2.y) - c.y;
+    const double ax = ((X0.x - X2.x) + (X1.x - X2.x)) * (1. / 6), ay = ((X0.y - X2.y) + (X1.y - X2.y)) * (1. / 6);
+    const double bx = ((X1.x - X0.x) + (X2.x - X0.x)) * (1. / 6), by = ((X1.y - X0.y) + (X2.y - X0.y)) * (1. / 6);
     reinterpret_cast<double2 *>(t.cell_q0)[at] = make_double2(ax * ia + ay * ib, ax * ib + ay * ic);
     reinterpret_cast<double2 *>(t.cell_q1)[at] = make_double2(bx * ia + by * ib, bx * ib + by * ic);
   }
