@@ -122,17 +122,18 @@ class _Watch:
     mesh's set-up) and go back with their solver."""
     PAGE = 1024
     _lock = threading.Lock()
-    _free = []       # (page, its host view, index)
+    _free = []       # (page, index)
 
     def __init__(self):
         with self._lock:
             if not self._free:
                 page = torch.zeros(self.PAGE, dtype=torch.int32, pin_memory=True)
-                self._free.extend((page, page.numpy(), k) for k in range(self.PAGE))
+                self._free.extend((page, k) for k in range(self.PAGE))
             slot = self._free.pop()
         weakref.finalize(self, self._give_back, slot)
-        self.page, self.seen, self.at = slot
-        self.seen[self.at] = 0
+        self.page, self.at = slot
+        self.late = ctypes.c_int32.from_address(self.page.data_ptr() + 4 * self.at)   # read on every call
+        self.late.value = 0
 
     @property
     def word(self):
@@ -146,11 +147,11 @@ class _Watch:
         """The tables ``t`` of a mesh for a solver that reports here."""
         own = type(t).from_buffer_copy(t)
         own.memory = t.memory
-        own.late = self.page.data_ptr() + 4 * self.at
+        own.late = ctypes.addressof(self.late)
         return own
 
     def check(self):
-        if self.seen[self.at]:
+        if self.late.value:
             raise _lib.MbError("a step on tiles waited in vain for its copies: the solver's state is not complete")
 
 
