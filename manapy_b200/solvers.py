@@ -628,12 +628,12 @@ class AdvectionDiffusionSolver:
         self._setup()
 
     def launches_per_step(self):
-        """Kernel launches of one fused step."""
+        """Kernel launches of one fused step from the cell array that is there now."""
         # (tetrahedra at order 2 through mb_advdiff_step pack rows first; the solver's steps
         # carry them from one step to the next instead; with the edge sums the first phase is
         # two launches: vertex and edge sums, then the cells)
         dm = self._dm
-        if dm is not None and self._tiles is not None:
+        if dm is not None and self._on_tiles(self.var._s.dev["cell"]):
             return 1 if self.dim == 2 else 2
         sums = dm is not None and self.order == 2 and dm.struct is not None and bool(dm.struct.cell_edges)
         return 1 + int(self.order == 2 or bool(self.diffusion)) + int(sums)
@@ -1151,9 +1151,10 @@ class ShallowWaterSolver:
         return float(ff.index_select(0, self._bfaces).double().sum().item())
 
     def launches_per_step(self):
-        """Kernel launches of one fused step: the step on tiles, or face fluxes and cells (+ next
-        dt); [gradients]."""
-        return (2 if self._tiles is None else 1) + int(self.order == 2)
+        """Kernel launches of one fused step from the arrays that are there now: the step on tiles, or
+        face fluxes and cells (+ next dt); [gradients]."""
+        on_tiles = self._on_tiles([var._s.dev["cell"] for var in self.varbs.values()])
+        return (1 if on_tiles else 2) + int(self.order == 2)
 
     def release_graphs(self):
         self._graphs.clear()
