@@ -671,12 +671,12 @@ class AdvectionDiffusionSolver:
                 g = self._get_graph(steps, depth)
                 if g is None:
                     break
-                a = self._graph_bufs[0]
+                a, b = self._graph_bufs
                 cur = var.dev("cell")
                 if cur is not a:        # a cell array installed since the capture
                     a.copy_(cur)
                     var.swap_cell(a)
-                    self._spare = self._graph_bufs[1]
+                self._spare = b         # which the replayed steps leave their last input in
                 if self._use_rows():
                     self._ensure_rows(a)         # the captured steps start from a's rows
                 g.replay()
