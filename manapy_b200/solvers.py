@@ -1392,14 +1392,15 @@ class EulerSolver:
         self._sync()
         n = int(n)
         D = self.GRAPH_DEPTH
+        key = (float(self.cfl), float(self.gamma))      # what a captured step holds besides the buffers
         while n > 0:
             if graph and n >= D and self._t % 6 == 0:
-                g = self._graphs.get("main")
+                g = self._graphs.get(key)
                 if g is None:
                     def body():
                         for k in range(D):
                             self._launch(k)
-                    g = self._graphs.capture("main", self._dm.device, body)
+                    g = self._graphs.capture(key, self._dm.device, body)
                 g.replay()
                 self._t += D
                 n -= D
