@@ -745,10 +745,11 @@ int mb_advdiff_step_noalloc(const mb_mesh *m, const mb_bc *bc, const mb_advdiff_
                             const double *w_in, double *w_out, const double *sign_cf,
                             const double *src, const double *dt_dev, void *stream);
 
-/* CUDA graphs of a solver's steps (no counterpart in manapy): mb_graph_begin makes a stream that captures
- * what is launched on it, on the current device; mb_graph_end ends the capture, gives the stream
- * back and the graph out (graph NULL: the capture is thrown away).  Launches of a graph on its
- * device as often as wanted, then mb_graph_free.  Any number of threads may capture at once. */
+/* CUDA graphs of a solver's steps (no counterpart in manapy): mb_graph_begin gives a stream that captures
+ * what is launched on it, on the current device; mb_graph_end (the same device current) ends the
+ * capture, takes the stream back and gives the graph out (graph NULL: the capture is thrown away).
+ * Launches of a graph on its device as often as wanted, then mb_graph_free.  Any number of threads may
+ * capture at once. */
 int mb_graph_begin(void **stream);
 int mb_graph_end(void *stream, void **graph);
 int mb_graph_launch(void *graph, void *stream);

@@ -1,9 +1,13 @@
 // CUDA graphs of a solver's steps (host code; no counterpart in manapy).
 //
-// A capture runs on a stream made for it: one from a pool that the program's other threads draw from
-// too could be theirs at the same time, and what they launch would become part of the graph.  The
-// mode is relaxed, so what other threads do meanwhile (allocate, free another graph) does not
-// invalidate the capture.  Nothing here is shared between captures, so threads need no lock.
+// A capture has a stream to itself while it runs: one from a pool that the program's other threads
+// draw from too could be theirs at the same time, and what they launch would become part of the
+// graph.  Streams are kept for later captures, as many a device as ever ran at once.  The mode is
+// relaxed, so what other threads do meanwhile (allocate, free another graph) does not invalidate
+// the capture.
+#include <mutex>
+#include <vector>
+
 #include "fv_common.cuh"
 
 using namespace mb;
@@ -16,6 +20,38 @@ struct Relaxed {
   Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
   ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
+
+struct Kept {
+  int device;
+  cudaStream_t stream;
+};
+std::mutex kept_lock;
+std::vector<Kept> &kept() {      // never destroyed: a thread may end its capture while the process exits
+  static auto *v = new std::vector<Kept>;
+  return *v;
+}
+cudaError_t take_stream(cudaStream_t *s) {
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  {
+    const std::lock_guard<std::mutex> hold(kept_lock);
+    for (size_t k = 0; k < kept().size(); ++k)
+      if (kept()[k].device == device) {
+        *s = kept()[k].stream;
+        kept()[k] = kept().back();
+        kept().pop_back();
+        return cudaSuccess;
+      }
+  }
+  return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+}
+void keep_stream(cudaStream_t s) {
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) return;
+  const std::lock_guard<std::mutex> hold(kept_lock);
+  kept().push_back(Kept{device, s});
+}
 }  // namespace
 
 extern "C" {
@@ -25,7 +61,7 @@ int mb_graph_begin(void **stream) {
   if (!stream) return MB_EINVAL;
   const Relaxed relaxed;
   cudaStream_t s = nullptr;
-  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return MB_ECUDA;
+  if (take_stream(&s) != cudaSuccess) return MB_ECUDA;
   if (cudaStreamBeginCapture(s, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
     cudaStreamDestroy(s);
     return MB_ECUDA;
@@ -44,7 +80,7 @@ int mb_graph_end(void *stream, void **graph) {
   cudaError_t e = cudaStreamEndCapture(s, &g);
   if (e == cudaSuccess && graph) e = cudaGraphInstantiate(&x, g, 0);
   if (g) cudaGraphDestroy(g);
-  cudaStreamDestroy(s);
+  if (e == cudaSuccess) keep_stream(s); else cudaStreamDestroy(s);
   if (graph) *graph = e == cudaSuccess ? x : nullptr;
   return e == cudaSuccess ? MB_OK : MB_ECUDA;
 }
