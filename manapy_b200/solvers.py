@@ -48,11 +48,12 @@ def _capturing():
 class _Graph:
     """A captured CUDA graph."""
 
-    def __init__(self, handle, device):
-        self.handle, self.device, self.free = handle, device, _lib.lib().mb_graph_free
+    def __init__(self, handle, index):
+        self.handle, self.index, self.free = handle, index, _lib.lib().mb_graph_free
 
     def replay(self):
-        _lib.call("mb_graph_launch", self.handle, torch.cuda.current_stream(self.device).cuda_stream)
+        # by index: torch takes 3 us to find that of a device's name
+        _lib.call("mb_graph_launch", self.handle, torch.cuda.current_stream(self.index).cuda_stream)
 
     def __del__(self):
         self.free(self.handle)      # a launch still running ends first
@@ -61,30 +62,36 @@ class _Graph:
 class _Graphs:
     """Captured CUDA graphs of a solver by key, the last few used."""
     MOST = 6
+    COST = 16                # steps
 
     def __init__(self):
         self.by_key = {}
-        self.seen = {}       # keys asked for once, the last MOST
+        self.asked = {}      # how often, of the last MOST keys asked for, with or without a graph
 
     def clear(self):
         self.by_key.clear()
-        self.seen.clear()
+        self.asked.clear()
 
     def get(self, key):
         g = self.by_key.pop(key, None)
         if g is not None:
             self.by_key[key] = g        # most recently used last
+            self._ask(key)
         return g
 
-    def worth(self, key):
-        """Whether a run of this key was asked for before: a capture costs about what launching its
-        steps one by one does, so a length seen once is not captured, nor one that comes back after
-        more others than graphs are kept: its graph would be gone before its next use."""
-        if self.seen.pop(key, False):
-            return True
-        self.seen[key] = True
-        self._trim(self.seen)
-        return False
+    def worth(self, key, steps=COST):
+        """Whether to capture a run of ``steps`` steps that has no graph.  A capture costs what launching
+        16 steps does beside launching its own (0.3 ms against 20 us a step), so a length is captured
+        when the steps launched for it before come to that: a program that stops there has lost no
+        more than it had spent.  A length that comes back after more others than graphs are kept
+        is not: its graph would be gone, or another's that is used before it."""
+        return self._ask(key) * steps >= self.COST
+
+    def _ask(self, key):
+        before = self.asked.pop(key, 0)
+        self.asked[key] = before + 1
+        self._trim(self.asked)
+        return before
 
     def keep(self, key, g):
         self.by_key[key] = g
@@ -101,6 +108,7 @@ class _Graphs:
         streams of a pool that other threads use."""
         stream, handle, done = ctypes.c_void_p(), ctypes.c_void_p(), False
         with torch.cuda.device(device):
+            index = torch.cuda.current_device()
             _lib.call("mb_graph_begin", ctypes.byref(stream))
             try:
                 with torch.cuda.stream(torch.cuda.ExternalStream(stream.value, device=device)):
@@ -109,7 +117,7 @@ class _Graphs:
             finally:
                 rc = _lib.lib().mb_graph_end(stream, ctypes.byref(handle) if done else None)
         _lib.check(rc, "mb_graph_end")
-        g = _Graph(handle, device)
+        g = _Graph(handle, index)
         self.keep(key, g)
         return g
 
@@ -704,7 +712,7 @@ class AdvectionDiffusionSolver:
             for steps in self._graph_runs(n, depth):
                 key = (steps, _p(src))
                 g = self._graphs.get(key)
-                if g is None and (steps == depth or self._graphs.worth(key)):
+                if g is None and (steps == depth or self._graphs.worth(key, steps)):
                     def body():
                         for k in range(steps):
                             self._call_f32c(k % 2, src, self._stream())
@@ -739,7 +747,7 @@ class AdvectionDiffusionSolver:
         src = self._source_ptr()
         key = (steps, src)
         g = self._graphs.get(key)
-        if g is not None or (steps != depth and not self._graphs.worth(key)):
+        if g is not None or (steps != depth and not self._graphs.worth(key, steps)):
             return g
         var = self.var
         if self._graph_bufs is None:
@@ -1168,7 +1176,8 @@ class ShallowWaterSolver:
         n = int(nsteps)
         # a length asked for before is replayed from a graph: after 4 k steps every buffer and the dt
         # ring are where they were.  Longer runs repeat a graph of GRAPH_STEPS
-        while n >= 4 and not _capturing():
+        graphs = n >= 4 and not _capturing()
+        while graphs and n >= 4:
             steps = min(n & ~3, self.GRAPH_STEPS)
             key = (steps,) + self._prime()
             g = self._graphs.get(key)
@@ -1179,7 +1188,7 @@ class ShallowWaterSolver:
                 def body(steps=steps):
                     for _ in range(steps):
                         self._fused_step()
-                if self._graphs.worth(key):
+                if self._graphs.worth(key, steps):
                     self._graphs.capture(key, self._dm.device, body).replay()
                 else:
                     body()
