@@ -350,7 +350,7 @@ int mb_advdiff_step_tile(const mb_mesh *m, const mb_tiles *t, const mb_bc *bc, c
 
 /* Tiles of a tetrahedral mesh for the second-order step: local cells of a tile are its own, then at
  * cells + e the outside cells ext[e] that share a vertex with them; local nodes and edges are
- * those of its cells.  Coordinates are relative to the centre of the tile's first cell. */
+ * those of its cells.  Coordinates are relative to the mean of the centres of the tile's cells. */
 #define MB_TET_TILE_MAX_CELLS 512
 typedef struct mb_tet_tiles {
   int32_t cells, count;          /* cells per tile (even, 32 .. MB_TET_TILE_MAX_CELLS), ceil(nbcells / cells) tiles */

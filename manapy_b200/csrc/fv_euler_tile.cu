@@ -8,10 +8,12 @@
 // of a cell alone (its sound speed, momentum and energy fluxes) is formed once per cell: 4 divisions
 // per face and 6 per cell instead of 18 per face.
 //
-// Measured (B200, per step in a CUDA graph, two launches -> this): 2M triangles 159 -> 141 us, 720,000
-// 62.5 -> 56, 45,000 8.8 -> 5.7, 1,800 7.3 -> 4.5.  The FP64 chains between barriers bound it (issue
-// slots 43 % busy, FP64 pipe 32 %, 18 warps per SM); other shapes at 720,000 cells: 192 threads x 4
-// blocks 57-60 us, 256 x 3 60, 96 x 7 59-61; without the per-cell pass 56 (256 cells).
+// Measured (B200, per step in CUDA graphs of 24, two launches -> this, one session): 2M triangles
+// 161 -> 141 us, 720,000 63.6 -> 60.6, 45,000 9.3 -> 5.8, 1,800 8.0 -> 4.6.  The latency of the FP64
+// chains between barriers bounds it (issue slots 46 % busy, FP64 pipe 35 %, 30 % of the warps:
+// registers and shared memory allow 5 blocks).  Other shapes at 720,000 cells, beside 56.6 us for
+// this one in the same session: 192 threads x 4 blocks 57-60 us, 256 x 3 60, 96 x 7 59-61; without the
+// per-cell pass 56 (256 cells).
 #include "fv_euler.cuh"
 #include "fv_tile.cuh"
 

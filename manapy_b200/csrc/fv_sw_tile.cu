@@ -8,9 +8,10 @@
 // faces once; a flux crosses shared memory only.  Faces between two tiles are evaluated by both
 // (a tenth more at 256 cells).  Same arithmetic, same bits (fv_sw.cuh).
 //
-// Measured (B200, per step in a CUDA graph, two launches -> this): 1.28M triangles 129 -> 80 us,
-// 245,000 26.5 -> 18.5, 80,000 11.8 -> 7.5, 45,000 9.2 -> 5.8, 5,000 7.3 -> 4.5; second order 45,000
-// 17.1 -> 15.8.  The passes are long serial chains of FP64 operations (square roots and divisions
+// Measured (B200, per step in a CUDA graph of 48, two launches -> this, one session): 1.28M triangles
+// 133 -> 80 us, 245,000 27.9 -> 19.4, 80,000 12.9 -> 7.4, 45,000 10.1 -> 5.8, 5,000 8.0 -> 4.6; second
+// order (three launches -> two) 1.28M 277 -> 233, 245,000 63.9 -> 48.1, 45,000 20.8 -> 14.3, 5,000
+// 17.5 -> 12.0.  The passes are long serial chains of FP64 operations (square roots and divisions
 // among them) between barriers, so many small blocks per SM do best: 1.28M triangles, 128 threads x
 // 5 blocks (96 registers) 80 us with 256-cell tiles; 128 x 6 93; 256 x 3 96; 160 x 4 87; 384 x 2 101.
 #include "fv_sw.cuh"

@@ -22,9 +22,9 @@
 //
 // Large meshes keep the sums in memory (k_tet_sums, k_tet_cell below) and take the same fluxes.
 //
-// Measured (B200, per step in a CUDA graph, three launches -> this): 2,058 tetrahedra 32 -> 15 us,
-// 16,464 34 -> 15.5, 48,000 39 -> 18.7, 93,750 50 -> 34; with the sums in memory 384,000 115 -> 81,
-// 1,572,864 372 -> 254.  k_tet_flux reads 208 B of DRAM per cell and takes 18 us at 384,000 cells
+// Measured (B200, per step in CUDA graphs of the tuned length, three launches -> this, one session):
+// 2,058 tetrahedra 38.9 -> 17.7 us, 16,464 43.2 -> 18.3, 48,000 45.5 -> 21.6, 93,750 47.4 -> 37.6; with
+// the sums in memory 384,000 125 -> 86, 1,572,864 389 -> 265.  k_tet_flux reads 208 B of DRAM per cell and takes 18 us at 384,000 cells
 // where k_f3_phase2 took 45.  The gradient pass is bound by its chain of passes and by reading the
 // cells around a tile (512 threads x 2 blocks; 384 x 2 100-118 us at 384,000 cells, 256 x 3 124).
 #include "fv_tile.cuh"

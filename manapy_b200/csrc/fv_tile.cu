@@ -14,9 +14,10 @@
 //      with static coefficients (k_tile_coef), forward Euler.
 // The face layer's cells are computed by each tile that needs them (a quarter more at 384 cells).
 //
-// Measured (B200, per step in a CUDA graph, two-launch step with tuned launch shapes -> this):
-// 2M triangles 187 -> 107 us, 500,000 48.5 -> 33, 180,000 21.4 -> 14.0, 62,658 13.8 -> 7.4, 1,152
-// 11.9 -> 6.2; first order with diffusion 20,000 8.8 -> 4.2; no diffusion 245,000 28 -> 15.
+// Measured (B200, per step in CUDA graphs of the tuned length, two-launch step with tuned launch shapes
+// -> this, one session): 2M triangles 188 -> 112 us, 500,000 48.7 -> 34.2, 180,000 21.6 -> 15.1,
+// 62,658 15.7 -> 8.0, 1,152 13.9 -> 6.8; first order with diffusion 20,000 10.2 -> 4.7; no diffusion
+// 245,000 27.3 -> 16.0.
 // It moves 225 B of DRAM per cell-update (500,000 cells).  What bounds it is the chain of passes in
 // a block (barriers 30 % of the stalls, bulk copies and smem latency most of the rest; the
 // load/store pipe is 45 % busy, two fifths of that bank conflicts), so three blocks per SM overlap
