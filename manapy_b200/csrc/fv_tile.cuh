@@ -231,10 +231,15 @@ template <class... P, class... A>
 inline cudaError_t tile_launch_ex(const cudaLaunchConfig_t &cfg, void (*k)(P...), A... args) {
   return cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
+// a refusal is reported by the call that met it, not again by the next one that asks for the last error
+inline cudaError_t tile_done(cudaError_t e) {
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
 template <auto K, class... A>
 inline cudaError_t tile_launch(int blocks, int threads, int bytes, cudaStream_t st, A... args) {
   if (bytes > 48 * 1024) {                       // what every kernel may take
-    const cudaError_t e = tile_shared_limit<K>();
+    const cudaError_t e = tile_done(tile_shared_limit<K>());
     if (e != cudaSuccess) return e;
   }
   cudaLaunchAttribute at[1];
@@ -247,7 +252,7 @@ inline cudaError_t tile_launch(int blocks, int threads, int bytes, cudaStream_t 
   cfg.stream = st;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return tile_launch_ex(cfg, K, args...);
+  return tile_done(tile_launch_ex(cfg, K, args...));
 }
 
 // flags of a cell record of the tiles with faces: bit j left cell of face j, bits 3-8 manapy's order of
