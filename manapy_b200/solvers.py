@@ -894,6 +894,7 @@ class ShallowWaterSolver:
             # step mins the next one into the slot after it (1e6 before) and resets the one after that
             self._dt_buf = torch.full((4,), 1e6, dtype=torch.float64, device=dev)
             self._dt_slots = [self._dt_buf[k:k + 1] for k in range(4)]
+            self._dt_ptrs = [t.data_ptr() for t in self._dt_slots]
             self._cur = 0
             self._dt_key = None
             self._tiles = self._dm.face_tiles(self._stream()) if self.precision == "fp64" else None
@@ -1039,23 +1040,29 @@ class ShallowWaterSolver:
         if self._spare is None:
             self._spare = [torch.empty_like(t) for t in qin]
         qout = self._spare
-        cur, nxt = self._use_dt(), self._slot(1)
-        q = _lib.p5([_p(t) for t in qin] + [_p(z)])
-        scratch = _p(self._scratch) if self._scratch is not None else None
-        options = self._options()
-        if self._on_tiles(qin + [z]):
-            _lib.call("mb_sw_step_tile", self._dm.struct, self._tiles, q, _lib.p4([_p(t) for t in qout]), *options,
-                      scratch, _p(cur), _p(nxt), _p(self._slot(2)), self._stream())
-            self._ff_step = options
-        else:
-            _lib.call("mb_sw_step_ex", self._dm.struct, q, _lib.p5([_p(t) for t in qout] + [_p(z)]), *options, scratch,
-                      _p(self._face_flux()), _p(cur), _p(nxt), self._stream())
-            self._slot(2).fill_(1e6)    # as the step on tiles leaves it
-            self._ff_step = None
+        self._use_dt()
+        self._ff_step = self._call_step(qin, z, qout, 0)
         self._spare = [self.varbs[k].swap_cell(t) for k, t in zip(names, qout)]
         self._cur = (self._cur + 1) % 4
         self._dt_key = self._state_key()
         self._dt_host = None
+
+    def _call_step(self, qin, z, qout, k):
+        """The launches of one FP64 step, whose dt is ``k`` slots after the current one; the options of a step
+        on tiles, None for one that stored its face fluxes."""
+        dt, at = self._dt_ptrs, self._cur + k
+        cur, nxt, after = dt[at % 4], dt[(at + 1) % 4], dt[(at + 2) % 4]
+        q, out, z = [t.data_ptr() for t in qin], [t.data_ptr() for t in qout], z.data_ptr()
+        scratch = _p(self._scratch)
+        options = self._options()
+        if self._tiles is not None and (q[0] | q[1] | q[2] | q[3] | z) % 16 == 0:      # _on_tiles()
+            _lib.call("mb_sw_step_tile", self._dm.struct, self._tiles, _lib.p5(q + [z]), _lib.p4(out), *options,
+                      scratch, cur, nxt, after, self._stream())
+            return options
+        _lib.call("mb_sw_step_ex", self._dm.struct, _lib.p5(q + [z]), _lib.p5(out + [z]), *options, scratch,
+                  _p(self._face_flux()), cur, nxt, self._stream())
+        self._dt_slots[(at + 2) % 4].fill_(1e6)            # as the step on tiles leaves it
+        return None
 
     # ------------------------------------------------------------ fp32c mode
     _NAMES = ("h", "hu", "hv", "hc", "Z")
@@ -1083,20 +1090,22 @@ class ShallowWaterSolver:
         return self._q32[self._q32_i], self._q32[2]
 
     def _fused_step_f32c(self):
-        qin, z = self._f32_state()
-        qout = self._q32[1 - self._q32_i]
-        cur = self._use_dt()
-        nxt = self._slot(1)
-        k0 = self._q32_i
-        _lib.call("mb_sw_step_f32c_ex", self._dm.struct, _lib.p5([_p(t) for t in qin] + [_p(z)]),
-                  _lib.p5([_p(t) for t in qout] + [_p(z)]), _lib.p4([_p(t) for t in self._lo32[k0]]),
-                  _lib.p4([_p(t) for t in self._lo32[1 - k0]]), float(self.cfl), float(self.grav), int(self.order),
-                  _lib.WALLS[self.walls], _p(self._ff32), _p(cur), _p(nxt), self._stream())
-        self._q32_i = 1 - k0
+        self._f32_state()
+        self._use_dt()
+        self._call_step_f32c(self._q32_i, 0)
+        self._q32_i = 1 - self._q32_i
         self._f32_publish()
         self._cur = (self._cur + 1) % 4
         self._dt_key = self._state_key()
         self._dt_host = None
+
+    def _call_step_f32c(self, i, k):
+        """The launches of one step from FP32 buffer ``i`` into the other (``k`` as in ``_call_step``)."""
+        z, dt, at = _p(self._q32[2]), self._dt_ptrs, self._cur + k
+        _lib.call("mb_sw_step_f32c_ex", self._dm.struct, _lib.p5([_p(t) for t in self._q32[i]] + [z]),
+                  _lib.p5([_p(t) for t in self._q32[1 - i]] + [z]), _lib.p4([_p(t) for t in self._lo32[i]]),
+                  _lib.p4([_p(t) for t in self._lo32[1 - i]]), *self._options(), _p(self._ff32), dt[at % 4],
+                  dt[(at + 1) % 4], self._stream())
 
     def _f32_publish(self):
         """Make the current FP32 state the variables' cell arrays (converted on first read)."""
@@ -1181,20 +1190,28 @@ class ShallowWaterSolver:
             steps = min(n & ~3, self.GRAPH_STEPS)
             key = (steps,) + self._prime()
             g = self._graphs.get(key)
+            if g is None and self._graphs.worth(key, steps):
+                g = self._graphs.capture(key, self._dm.device, lambda: self._call_steps(steps))
             if g is not None:
                 g.replay()
                 self._published()
             else:
-                def body(steps=steps):
-                    for _ in range(steps):
-                        self._fused_step()
-                if self._graphs.worth(key, steps):
-                    self._graphs.capture(key, self._dm.device, body).replay()
-                else:
-                    body()
+                for _ in range(steps):
+                    self._fused_step()
             n -= steps
         for _ in range(n):
             self._fused_step()
+
+    def _call_steps(self, steps):
+        """The launches of ``steps`` steps (a multiple of 4) from the primed state, and nothing else: the state
+        is the solver's own until they run, whatever interrupts a capture of them."""
+        if self.precision == "fp32c":
+            for k in range(steps):
+                self._call_step_f32c((self._q32_i + k) % 2, k)
+            return
+        q, z = [self.varbs[k].dev("cell") for k in ("h", "hu", "hv", "hc")], self.Z.dev("cell")
+        for k in range(steps):
+            self._call_step(*((q, z, self._spare) if k % 2 == 0 else (self._spare, z, q)), k)
 
     def _prime(self):
         """All that a step does besides its launches (uploads of host edits, buffers, the dt of the
