@@ -49,11 +49,14 @@ class _Graph:
     """A captured CUDA graph."""
 
     def __init__(self, handle, index):
-        self.handle, self.index, self.free = handle, index, _lib.lib().mb_graph_free
+        self.handle, self.index = handle, index
+        self.launch, self.free = _lib.lib().mb_graph_launch, _lib.lib().mb_graph_free
 
     def replay(self):
-        # by index: torch takes 3 us to find that of a device's name
-        _lib.call("mb_graph_launch", self.handle, torch.cuda.current_stream(self.index).cuda_stream)
+        # the raw stream, as Triton's launcher asks for it: torch.cuda.current_stream() takes 1-4 us
+        rc = self.launch(self.handle, torch._C._cuda_getCurrentRawStream(self.index))
+        if rc != _lib.MB_OK:
+            _lib.check(rc, "mb_graph_launch")
 
     def __del__(self):
         self.free(self.handle)      # a launch still running ends first
@@ -76,7 +79,10 @@ class _Graphs:
         g = self.by_key.pop(key, None)
         if g is not None:
             self.by_key[key] = g        # most recently used last
-            self._ask(key)
+            self.asked.pop(key, None)
+            self.asked[key] = 1
+            if len(self.asked) > self.MOST:
+                self._trim(self.asked)
         return g
 
     def worth(self, key, steps=COST):
