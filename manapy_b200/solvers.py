@@ -128,6 +128,9 @@ class _Graphs:
         return g
 
 
+_NOT_LATE = ctypes.c_int32(0)      # the word of a solver without tiles
+
+
 class _Watch:
     """A word in pinned memory that a step on tiles sets when a wait for its copies ran out (its limit is
     seconds: a fault of the machine, never seen).  The state is not a step's from there on.
@@ -276,11 +279,11 @@ class AdvectionDiffusionSolver:
         self._sign32_key = None
         self._src32 = None
         self._src32_key = None
-        self._watch = None
+        self._watch, self._late = None, _NOT_LATE
 
     # ------------------------------------------------------------ device helpers
     def _setup(self):
-        if self._watch is not None:
+        if self._late.value:
             self._watch.check()
         if self._dm is None:
             self._dm = self.domain.device_mesh
@@ -315,6 +318,7 @@ class AdvectionDiffusionSolver:
                               self.var.device_bc.struct, self._params, _p(self._coef), self._stream())
             if self._tiles is not None:
                 self._watch = _Watch()
+                self._late = self._watch.late
                 self._tiles = self._watch.tiles(self._tiles)
         return self._dm
 
@@ -881,7 +885,7 @@ class ShallowWaterSolver:
         self.signature = self.domain.signature
         self._dm = None
         self._tiles = None
-        self._watch = None
+        self._watch, self._late = None, _NOT_LATE
         self._ff = None
         self._ff_step = None   # _options() of the last one-launch step, whose face fluxes are not kept
         self._graphs = _Graphs()
@@ -891,7 +895,7 @@ class ShallowWaterSolver:
         self._fused = False
 
     def _setup(self):
-        if self._watch is not None:
+        if self._late.value:
             self._watch.check()
         if self._dm is None:
             self._dm = self.domain.device_mesh
@@ -906,6 +910,7 @@ class ShallowWaterSolver:
             self._tiles = self._dm.face_tiles(self._stream()) if self.precision == "fp64" else None
             if self._tiles is not None:
                 self._watch = _Watch()
+                self._late = self._watch.late
                 self._tiles = self._watch.tiles(self._tiles)
             if self.order == 2:
                 self._scratch = torch.zeros(5 * self._dm.nbcells, dtype=torch.float64, device=dev)
@@ -1295,12 +1300,12 @@ class EulerSolver:
         self.dt = float(get("dt"))
         self.backend = self.domain.backend
         self._dm = None
-        self._watch = None
+        self._watch, self._late = None, _NOT_LATE
         self._graphs = _Graphs()
 
     # ------------------------------------------------------------ state
     def _setup(self):
-        if self._watch is not None:
+        if self._late.value:
             self._watch.check()
         if self._dm is None:
             for k, v in self.varbs.items():
@@ -1317,6 +1322,7 @@ class EulerSolver:
             self._tiles = dm.face_tiles(self._stream(), dm.face_tile_cells(dm.nbcells, dm.EULER_TILE_CELLS))
             if self._tiles is not None:
                 self._watch = _Watch()
+                self._late = self._watch.late
                 self._tiles = self._watch.tiles(self._tiles)
             else:
                 # the two-launch step: face fluxes, and its static tables (face records, left-cell bits)
